@@ -71,12 +71,12 @@ def _compile(cmd: List[str], out: str, log: str) -> str:
 # Sources of a library that holds one model family's kernels only (``build_cuda(part=...)``): a first start
 # on a fresh checkout compiles what that family needs.
 PARTS = {
-    "latent": ["elementwise", "gemm_tcgen05", "gemm_f32", "norm_conv", "latent_attention", "attention_tc", "sampling"],
-    "layered": ["elementwise", "gemm_tcgen05", "gemm_f32", "norm_conv", "residual_norm", "latent_attention",
+    "latent": ["elementwise", "gemm_tcgen05", "gemm_stream", "gemm_f32", "norm_conv", "latent_attention", "attention_tc", "sampling"],
+    "layered": ["elementwise", "gemm_tcgen05", "gemm_stream", "gemm_f32", "norm_conv", "residual_norm", "latent_attention",
                 "attention_tc", "linear_attention", "moe", "sampling"],
-    "heads": ["elementwise", "gemm_tcgen05", "gemm_f32", "norm_conv", "residual_norm", "rope_kv", "attention",
+    "heads": ["elementwise", "gemm_tcgen05", "gemm_stream", "gemm_f32", "norm_conv", "residual_norm", "rope_kv", "attention",
               "attention_f32", "attention_tc", "moe", "sampling"],
-    "pair": ["elementwise", "gemm_tcgen05", "gemm_f32", "norm_conv", "residual_norm", "rope_kv", "attention",
+    "pair": ["elementwise", "gemm_tcgen05", "gemm_stream", "gemm_f32", "norm_conv", "residual_norm", "rope_kv", "attention",
              "attention_f32", "attention_tc", "attention_talk", "linear_attention", "selective_scan", "moe", "sampling"],
 }
 

@@ -63,7 +63,7 @@ class ParallelLMHead(BaseOP):
     def forward_local(self, x: torch.Tensor) -> torch.Tensor:
         """fp32 logits of this rank's vocabulary shard ``[rows, ceil(V / tp)]`` (columns past the
         shard's length are padding)."""
-        return ops.gemm(x, self._w, None, torch.float32)
+        return ops.logits(x, self._w)
 
     def gather(self, local: torch.Tensor) -> torch.Tensor:
         """Shard logits → full-vocabulary logits ``[rows, V]`` on every rank."""

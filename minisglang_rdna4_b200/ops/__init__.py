@@ -154,6 +154,13 @@ def gemm(x, w, bias=None, out_dtype: Optional[torch.dtype] = None):
     return ref.gemm(x, w, bias, out_dtype)
 
 
+def logits(x, w):
+    """fp32 ``x @ w.T`` for the rows that a step samples."""
+    if x.is_cuda:
+        return _cuda().logits(x, w)
+    return ref.gemm(x, w, None, torch.float32)
+
+
 def gemm_w8a8(x_q, x_scale, w_q, w_scale, out_dtype=torch.bfloat16, bias=None):
     if x_q.is_cuda:
         return _cuda().gemm_w8a8(x_q, x_scale, w_q, w_scale, out_dtype, bias)

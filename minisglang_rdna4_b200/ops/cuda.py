@@ -689,7 +689,74 @@ def take_pending_gemm_tp():
     return args
 
 
-def _gemm(kind, a, b, n, k, out_dtype, a_scale=None, b_scale=None, bias=None, sf_atoms=None, bn=0, max_ctas=0):
+_STREAM_PLANS: Dict[Tuple[int, int, int, bool], Tuple[int, int]] = {}
+_STREAM_COUNTERS: Dict[Tuple, list] = {}
+STREAM_PLANES = 8
+
+
+def _stream_plan(kind: int, n: int, k: int, planes: bool) -> Tuple[int, int]:
+    """(CTAs, planes) of ``csrc/gemm_stream.cu`` for a weight matrix."""
+    key = (kind, n, k, planes)
+    got = _STREAM_PLANS.get(key)
+    if got is None:
+        most = ctypes.c_int()
+        ctas = int(lib().msgl_gemm_stream_plan(kind, n, k, STREAM_PLANES if planes else 0, ctypes.addressof(most)))
+        got = _STREAM_PLANS[key] = (ctas, most.value)
+    return got
+
+
+def _stream_counters(device, tiles: int) -> torch.Tensor:
+    """Arrival counters of the tiles that CTAs share: zero between calls. One set for each stream, and one for what is
+    captured on it, since calls on two streams may run side by side. A captured graph holds their address, so they stay
+    (16 KB each; streams come from a pool of fixed size)."""
+    key = (device, _stream(), torch.cuda.is_current_stream_capturing())
+    sets = _STREAM_COUNTERS.setdefault(key, [])
+    if not sets or sets[-1].numel() < tiles:
+        sets.append(workspace(f"GEMM tile counters {key[1:]} {len(sets)}", max(2 * tiles, 4096), torch.int32, device, zero=True))
+    return sets[-1]
+
+
+def _stream_pays(m: int, weight_bytes: int, planes: bool) -> bool:
+    """Whether ``csrc/gemm_stream.cu`` is the faster one. Unreduced sums: up to 128 rows (B200, K = 12288 of 4096 16-bit
+    columns: 21.7 against 31 us at 64 rows; at 256 its eight planes cost the next norm what the product gains). Finished
+    sums: tiles that CTAs share are summed by one of them, about 4 us and 0.05 us a row, which up to 32 rows the even deal
+    always makes up for (6144 x 2560 in 4 bits: 10.0 against 12.2 us at 16 rows, 14.5 against 10.4 at 64), up to 64 rows
+    where there are enough bytes to deal (24576 x 4096 in 16 bits: 42.7 against 48.7 us at 64 rows, 52 against 51 at 128)."""
+    if planes:
+        return m <= 128
+    return m <= 32 or (m <= 64 and weight_bytes >= 48 << 20)
+
+
+def _decode_step() -> bool:
+    """Whether the step that runs is a decode step: its rows are one per request, so nothing asks that they come out bit for
+    bit as the same rows of a longer chunk would (``SPLIT_K_DECODE`` off: verification rows have to)."""
+    from ..core import try_global_ctx
+
+    ctx = try_global_ctx()
+    batch = ctx._batch if ctx is not None else None
+    return SPLIT_K_DECODE and batch is not None and batch.is_decode and not batch.spec_verify
+
+
+def _gemm_stream(kind, a, b, m, n, k, out_dtype, a_scale, b_scale, bias, sf_atoms, want_planes):
+    ctas, most = _stream_plan(kind, n, k, want_planes)
+    ws = count = None
+    if want_planes:
+        out = torch.empty((most, m, n), dtype=torch.float32, device=a.device)
+    else:
+        most = 0
+        out = torch.empty((m, n), dtype=out_dtype, device=a.device)
+        columns = next(c for c in (16, 32, 64, 128) if m <= c)
+        ws = torch.empty(2 * ctas * columns * 128, dtype=torch.float32, device=a.device)
+        count = _stream_counters(a.device, (n + 127) // 128)
+    check(lib().msgl_gemm_stream(kind, _p(a), a.stride(0), _p(b), _p(out), n, m, n, k, _p(a_scale), _p(b_scale), _p(bias),
+                                 _DT[bias.dtype] if bias is not None else 0, _p(sf_atoms),
+                                 _DT[torch.float32 if want_planes else out_dtype], most, ctas, _p(ws), _p(count), _stream()),
+          "gemm_stream")
+    _count(("gemm_f16", "gemm_bf16", "gemm_w8a8", "gemm_w4a8_mxfp4")[kind] + "_stream", "gemm_stream_kernel")
+    return SplitPartial(out, out_dtype) if want_planes else out
+
+
+def _gemm(kind, a, b, n, k, out_dtype, a_scale=None, b_scale=None, bias=None, sf_atoms=None, bn=0, max_ctas=0, few=False):
     assert a.dim() == 2 and a.stride(1) == 1 and b.is_contiguous()
     m = a.shape[0]
     tp = take_pending_gemm_tp()
@@ -704,6 +771,9 @@ def _gemm(kind, a, b, n, k, out_dtype, a_scale=None, b_scale=None, bias=None, sf
         return out
     global _PENDING_PLANES
     want_planes, _PENDING_PLANES = _PENDING_PLANES, False
+    if (0 < m <= 128 and bn == 0 and not max_ctas and not SPLIT_K and _stream_pays(m, b.nbytes, want_planes)
+            and (few or _decode_step())):
+        return _gemm_stream(kind, a, b, m, n, k, out_dtype, a_scale, b_scale, bias, sf_atoms, want_planes)
     if want_planes and 0 < m <= 256 and bn == 0:
         splits = _splitk_plan(kind, n, k)
         if splits > 1:
@@ -736,7 +806,13 @@ def _gemm(kind, a, b, n, k, out_dtype, a_scale=None, b_scale=None, bias=None, sf
     return out
 
 
-def gemm(x, w, bias=None, out_dtype=None, bn=0, max_ctas=0):
+def logits(x, w):
+    """fp32 ``x @ w.T`` for the rows that a step samples (a draft's verification: ``SPLIT_K_DECODE`` is off)."""
+    return gemm(x, w, None, torch.float32, few=SPLIT_K_DECODE)
+
+
+def gemm(x, w, bias=None, out_dtype=None, bn=0, max_ctas=0, few=False):
+    """``few``: the rows are no chunk of a prompt, whose results may not depend on how it was cut."""
     shape = x.shape
     x2 = x.reshape(-1, shape[-1])
     if x2.stride(1) != 1:
@@ -751,7 +827,7 @@ def gemm(x, w, bias=None, out_dtype=None, bn=0, max_ctas=0):
     n, k = w.shape
     if n % 8:
         raise ValueError("gemm: N must be a multiple of 8")
-    out = _gemm(kind, x2, w, n, k, out_dtype or x.dtype, bias=bias, bn=bn, max_ctas=max_ctas)
+    out = _gemm(kind, x2, w, n, k, out_dtype or x.dtype, bias=bias, bn=bn, max_ctas=max_ctas, few=few)
     if isinstance(out, SplitPartial):
         return out
     return out.view(*shape[:-1], n) if out is not None else None
@@ -890,7 +966,8 @@ def gemm_w4a16_status(reset=True) -> int:
 
 
 def gemm_status(reset=True) -> int:
-    return int(lib().msgl_gemm_status(int(reset)))
+    stream, tiled = int(lib().msgl_gemm_stream_status(int(reset))), int(lib().msgl_gemm_status(int(reset)))
+    return stream or tiled
 
 
 def gemm_pair_mode(mode: int) -> int:
