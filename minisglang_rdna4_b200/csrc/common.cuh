@@ -47,14 +47,16 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_float<__nv_bfloat16>(f
 template <> __device__ __forceinline__ __half from_float<__half>(float x) { return __float2half_rn(x); }
 template <> __device__ __forceinline__ float from_float<float>(float x) { return x; }
 
-template <typename T> __device__ __forceinline__ void load8(const T* p, float (&out)[8]) {
-  Vec8<T> v = *reinterpret_cast<const Vec8<T>*>(p);
+template <typename T> __device__ __forceinline__ void unpack8(const Vec8<T>& v, float (&out)[8]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     float2 f = to_float2(v.v[i]);
     out[2 * i] = f.x;
     out[2 * i + 1] = f.y;
   }
+}
+template <typename T> __device__ __forceinline__ void load8(const T* p, float (&out)[8]) {
+  unpack8(*reinterpret_cast<const Vec8<T>*>(p), out);
 }
 template <typename T> __device__ __forceinline__ void store8(T* p, const float (&in)[8]) {
   Vec8<T> v;

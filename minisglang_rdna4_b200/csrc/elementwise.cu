@@ -58,54 +58,90 @@ MSGL_API int msgl_embedding(const void* ids, const void* w, void* out, int rows,
 }
 
 // ------------------------------------------------------------------------------------------
-// RMSNorm family. One CTA of 128 threads per row; every thread keeps its VPT 16-byte vectors of
-// the (summed) row in registers between the reduction and the write, so the row is read once.
+// RMSNorm family. One CTA per row; every thread keeps its VPT 16-byte vectors of the (summed) row in
+// registers between the reduction and the write, so the row is read once.
 //   ADD   : residual += x (stored back, rounded to T), norm of the sum
 //   QUANT : emit e4m3 row + fp32 scale (amax/448) instead of T
-// ------------------------------------------------------------------------------------------
-constexpr int kRowThreads = 128;
-
 //   PLANES: x is fp32 [planes][rows][hidden], the K ranges of a split-K GEMM; they are summed in
 //           ascending order and rounded to T, which is what an unsplit GEMM would have handed over
-template <typename T, bool ADD, bool QUANT, int VPT, bool PLANES = false>
-__global__ void __launch_bounds__(kRowThreads) rms_norm_kernel(const T* __restrict__ x, T* __restrict__ residual,
-                                                               const T* __restrict__ w, T* __restrict__ out,
-                                                               uint8_t* __restrict__ out_q,
-                                                               float* __restrict__ out_scale, int hidden, float eps,
-                                                               float w_offset, int planes = 0,
-                                                               size_t plane_stride = 0) {
+//
+// Bound: HBM for many rows, one memory round trip for few. All loads of a row (x, residual, weight; of
+// planes four at a time) are issued before the first store: with the residual's store between two
+// vectors' loads each of up to eight vectors cost a round trip of its own. Threads and vectors a thread are
+// chosen by the width alone (never by the row count: the order of the sum, and with it a row's bits,
+// would follow), two vectors a thread, so that a decode step's few rows have all their bytes under way too.
+// B200, us, with the residual and e4m3 out, before -> after: 1 x 2560 3.9 -> 2.7, 64 x 4096 4.7 -> 3.1, 8190 x 2560 31.5 -> 30.3,
+// 8192 x 8192 120 -> 110 (4.3 TB/s); 5 planes of 64 x 4096 7.6 -> 4.5, 3 of 32 x 8192 11.9 -> 4.9.
+// ------------------------------------------------------------------------------------------
+template <typename T, bool ADD, bool QUANT, int VPT, int MAXT, bool PLANES = false>
+__global__ void __launch_bounds__(MAXT) rms_norm_kernel(const T* __restrict__ x, T* __restrict__ residual,
+                                                        const T* __restrict__ w, T* __restrict__ out,
+                                                        uint8_t* __restrict__ out_q, float* __restrict__ out_scale,
+                                                        int hidden, float eps, float w_offset, int planes,
+                                                        size_t plane_stride) {
   pdl_enter();
   __shared__ float scratch[32];
-  const int row = blockIdx.x;
-  const T* xr = x + (size_t)row * hidden;
-  const float* xp = reinterpret_cast<const float*>(x) + (size_t)row * hidden;
-  T* rr = ADD ? residual + (size_t)row * hidden : nullptr;
+  const int row = blockIdx.x, step = blockDim.x * 8;
+  const size_t at = (size_t)row * hidden;
   float v[VPT][8];
+  Vec8<T> xv[VPT], rv[VPT], wv[VPT];
+#pragma unroll
+  for (int j = 0; j < VPT; ++j) {
+    const int i = j * step + threadIdx.x * 8;
+    if (i < hidden) {
+      if (!PLANES) xv[j] = *reinterpret_cast<const Vec8<T>*>(x + at + i);
+      if (ADD) rv[j] = *reinterpret_cast<const Vec8<T>*>(residual + at + i);
+      wv[j] = *reinterpret_cast<const Vec8<T>*>(w + i);
+    }
+  }
+  if (PLANES) {
+    const float* xp = reinterpret_cast<const float*>(x) + at;
+#pragma unroll
+    for (int j = 0; j < VPT; ++j)
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[j][k] = 0.f;
+#pragma unroll 1
+    for (int p0 = 0; p0 < planes; p0 += 4) {
+      float4 t[4][VPT][2];
+#pragma unroll
+      for (int p = 0; p < 4; ++p)
+#pragma unroll
+        for (int j = 0; j < VPT; ++j) {
+          const int i = j * step + threadIdx.x * 8;
+          if (p0 + p < planes && i < hidden) {
+            t[p][j][0] = __ldg(reinterpret_cast<const float4*>(xp + (p0 + p) * plane_stride + i));
+            t[p][j][1] = __ldg(reinterpret_cast<const float4*>(xp + (p0 + p) * plane_stride + i + 4));
+          }
+        }
+#pragma unroll
+      for (int p = 0; p < 4; ++p)
+#pragma unroll
+        for (int j = 0; j < VPT; ++j)
+          if (p0 + p < planes && j * step + threadIdx.x * 8 < hidden)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              v[j][4 * h] += t[p][j][h].x; v[j][4 * h + 1] += t[p][j][h].y;
+              v[j][4 * h + 2] += t[p][j][h].z; v[j][4 * h + 3] += t[p][j][h].w;
+            }
+    }
+  }
   float ss = 0.f;
 #pragma unroll
   for (int j = 0; j < VPT; ++j) {
-    const int i = (j * kRowThreads + threadIdx.x) * 8;
+    const int i = j * step + threadIdx.x * 8;
     if (i < hidden) {
       if (PLANES) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) v[j][k] = 0.f;
-        for (int p = 0; p < planes; ++p) {
-          const float4 lo = __ldg(reinterpret_cast<const float4*>(xp + p * plane_stride + i));
-          const float4 hi = __ldg(reinterpret_cast<const float4*>(xp + p * plane_stride + i + 4));
-          v[j][0] += lo.x; v[j][1] += lo.y; v[j][2] += lo.z; v[j][3] += lo.w;
-          v[j][4] += hi.x; v[j][5] += hi.y; v[j][6] += hi.z; v[j][7] += hi.w;
-        }
-#pragma unroll
         for (int k = 0; k < 8; ++k) v[j][k] = to_float(from_float<T>(v[j][k]));
       } else {
-        load8(xr + i, v[j]);
+        unpack8(xv[j], v[j]);
       }
       if (ADD) {
         float r[8];
-        load8(rr + i, r);
+        unpack8(rv[j], r);
 #pragma unroll
         for (int k = 0; k < 8; ++k) v[j][k] += r[k];
-        store8(rr + i, v[j]);
+        store8(residual + at + i, v[j]);
         // the norm sees the rounded residual, exactly what the next layer will read
 #pragma unroll
         for (int k = 0; k < 8; ++k) v[j][k] = to_float(from_float<T>(v[j][k]));
@@ -119,17 +155,17 @@ __global__ void __launch_bounds__(kRowThreads) rms_norm_kernel(const T* __restri
   float amax = 0.f;
 #pragma unroll
   for (int j = 0; j < VPT; ++j) {
-    const int i = (j * kRowThreads + threadIdx.x) * 8;
+    const int i = j * step + threadIdx.x * 8;
     if (i < hidden) {
-      float wv[8];
-      load8(w + i, wv);
+      float wf[8];
+      unpack8(wv[j], wf);
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         // round to T as the unfused op would, so the quantised row matches norm -> quant
-        v[j][k] = to_float(from_float<T>(v[j][k] * rstd * (wv[k] + w_offset)));
+        v[j][k] = to_float(from_float<T>(v[j][k] * rstd * (wf[k] + w_offset)));
         if (QUANT) amax = fmaxf(amax, fabsf(v[j][k]));
       }
-      if (!QUANT) store8(out + (size_t)row * hidden + i, v[j]);
+      if (!QUANT) store8(out + at + i, v[j]);
     }
   }
   if (QUANT) {
@@ -138,65 +174,48 @@ __global__ void __launch_bounds__(kRowThreads) rms_norm_kernel(const T* __restri
     if (threadIdx.x == 0) out_scale[row] = scale;
 #pragma unroll
     for (int j = 0; j < VPT; ++j) {
-      const int i = (j * kRowThreads + threadIdx.x) * 8;
-      if (i < hidden) *reinterpret_cast<uint2*>(out_q + (size_t)row * hidden + i) = pack8_e4m3(v[j], scale);
+      const int i = j * step + threadIdx.x * 8;
+      if (i < hidden) *reinterpret_cast<uint2*>(out_q + at + i) = pack8_e4m3(v[j], scale);
     }
   }
 }
 
-template <typename T, int VPT>
-static void launch_rms_vpt(const void* x, void* residual, const void* w, void* out, void* out_q, void* out_scale,
+constexpr int kMaxRow = 16384, kMaxPlanesRow = 8192;   // widest row of a norm, and of one that sums planes
+
+// planes == 0: x is of type T
+template <typename T, int VPT, int MAXT>
+static void launch_rms_vpt(const void* x, int planes, void* residual, const void* w, void* out, void* out_q, void* out_scale,
                            int rows, int hidden, float eps, float off, cudaStream_t s) {
   const bool add = residual != nullptr, quant = out_q != nullptr;
-#define RMS_LAUNCH(A, Q)                                                                                    \
-  msgl_launch(rms_norm_kernel<T, A, Q, VPT>, dim3(rows), dim3(kRowThreads), 0, s, (const T*)x, (T*)residual, (const T*)w, (T*)out, \
-                                                            (uint8_t*)out_q, (float*)out_scale, hidden, eps, off, 0, (size_t)0)
-  if (add && quant) RMS_LAUNCH(true, true);
-  else if (add) RMS_LAUNCH(true, false);
-  else if (quant) RMS_LAUNCH(false, true);
-  else RMS_LAUNCH(false, false);
+  const int vecs = hidden / 8, threads = vecs > 0 ? ((vecs + VPT - 1) / VPT + 31) / 32 * 32 : 32;
+  const size_t stride = (size_t)rows * hidden;
+#define RMS_LAUNCH(A, Q, P)                                                                                                   \
+  msgl_launch(rms_norm_kernel<T, A, Q, VPT, MAXT, P>, dim3(rows), dim3(threads), 0, s, (const T*)x, (T*)residual, (const T*)w, \
+              (T*)out, (uint8_t*)out_q, (float*)out_scale, hidden, eps, off, planes, stride)
+  if constexpr (MAXT * VPT * 8 <= kMaxPlanesRow) {
+    if (planes > 0) {
+      if (quant) RMS_LAUNCH(true, true, true);
+      else RMS_LAUNCH(true, false, true);
+      return;
+    }
+  }
+  if (add && quant) RMS_LAUNCH(true, true, false);
+  else if (add) RMS_LAUNCH(true, false, false);
+  else if (quant) RMS_LAUNCH(false, true, false);
+  else RMS_LAUNCH(false, false, false);
 #undef RMS_LAUNCH
 }
 
 template <typename T>
-static int launch_rms(const void* x, void* residual, const void* w, void* out, void* out_q, void* out_scale,
-                      int rows, int hidden, float eps, int plus_one, cudaStream_t s) {
+static int launch_rms(const void* x, int planes, void* residual, const void* w, void* out, void* out_q, void* out_scale, int rows,
+                      int hidden, float eps, int plus_one, cudaStream_t s) {
   const float off = plus_one ? 1.f : 0.f;
-  const int vpt = (hidden / 8 + kRowThreads - 1) / kRowThreads;
-  if (vpt <= 1) launch_rms_vpt<T, 1>(x, residual, w, out, out_q, out_scale, rows, hidden, eps, off, s);
-  else if (vpt <= 2) launch_rms_vpt<T, 2>(x, residual, w, out, out_q, out_scale, rows, hidden, eps, off, s);
-  else if (vpt <= 3) launch_rms_vpt<T, 3>(x, residual, w, out, out_q, out_scale, rows, hidden, eps, off, s);
-  else if (vpt <= 4) launch_rms_vpt<T, 4>(x, residual, w, out, out_q, out_scale, rows, hidden, eps, off, s);
-  else if (vpt <= 6) launch_rms_vpt<T, 6>(x, residual, w, out, out_q, out_scale, rows, hidden, eps, off, s);
-  else if (vpt <= 8) launch_rms_vpt<T, 8>(x, residual, w, out, out_q, out_scale, rows, hidden, eps, off, s);
-  else if (vpt <= 16) launch_rms_vpt<T, 16>(x, residual, w, out, out_q, out_scale, rows, hidden, eps, off, s);
-  else return MSGL_BAD_ARG;
+  const int vecs = hidden / 8;
+  if (vecs <= 128) launch_rms_vpt<T, 1, 128>(x, planes, residual, w, out, out_q, out_scale, rows, hidden, eps, off, s);
+  else if (vecs <= 512) launch_rms_vpt<T, 2, 256>(x, planes, residual, w, out, out_q, out_scale, rows, hidden, eps, off, s);
+  else if (vecs <= 1024) launch_rms_vpt<T, 2, 512>(x, planes, residual, w, out, out_q, out_scale, rows, hidden, eps, off, s);
+  else launch_rms_vpt<T, 2, 1024>(x, planes, residual, w, out, out_q, out_scale, rows, hidden, eps, off, s);
   MSGL_CHECK_LAUNCH("rms_norm");
-  return MSGL_OK;
-}
-
-template <typename T, int VPT>
-static void launch_rms_planes_vpt(const void* x, int planes, void* residual, const void* w, void* out, void* out_q,
-                                  void* out_scale, int rows, int hidden, float eps, float off, cudaStream_t s) {
-  const size_t stride = (size_t)rows * hidden;
-  if (out_q != nullptr)
-    msgl_launch(rms_norm_kernel<T, true, true, VPT, true>, dim3(rows), dim3(kRowThreads), 0, s, (const T*)x, (T*)residual, (const T*)w, (T*)out, (uint8_t*)out_q, (float*)out_scale, hidden, eps, off, planes, stride);
-  else
-    msgl_launch(rms_norm_kernel<T, true, false, VPT, true>, dim3(rows), dim3(kRowThreads), 0, s, (const T*)x, (T*)residual, (const T*)w, (T*)out, (uint8_t*)out_q, (float*)out_scale, hidden, eps, off, planes, stride);
-}
-
-template <typename T>
-static int launch_rms_planes(const void* x, int planes, void* residual, const void* w, void* out, void* out_q,
-                             void* out_scale, int rows, int hidden, float eps, int plus_one, cudaStream_t s) {
-  const float off = plus_one ? 1.f : 0.f;
-  const int vpt = (hidden / 8 + kRowThreads - 1) / kRowThreads;
-  if (vpt <= 1) launch_rms_planes_vpt<T, 1>(x, planes, residual, w, out, out_q, out_scale, rows, hidden, eps, off, s);
-  else if (vpt <= 2) launch_rms_planes_vpt<T, 2>(x, planes, residual, w, out, out_q, out_scale, rows, hidden, eps, off, s);
-  else if (vpt <= 3) launch_rms_planes_vpt<T, 3>(x, planes, residual, w, out, out_q, out_scale, rows, hidden, eps, off, s);
-  else if (vpt <= 4) launch_rms_planes_vpt<T, 4>(x, planes, residual, w, out, out_q, out_scale, rows, hidden, eps, off, s);
-  else if (vpt <= 8) launch_rms_planes_vpt<T, 8>(x, planes, residual, w, out, out_q, out_scale, rows, hidden, eps, off, s);
-  else return MSGL_BAD_ARG;
-  MSGL_CHECK_LAUNCH("rms_norm_planes");
   return MSGL_OK;
 }
 
@@ -205,14 +224,12 @@ static int launch_rms_planes(const void* x, int planes, void* residual, const vo
 MSGL_API int msgl_rms_norm_planes(const void* x_planes, int planes, void* residual, const void* w, void* out,
                                   void* out_q, void* out_scale, int rows, int hidden, float eps, int plus_one,
                                   int dtype, cudaStream_t stream) {
-  if (hidden % 8 || hidden > 8 * 8 * kRowThreads || planes < 1 || residual == nullptr) return MSGL_BAD_ARG;
+  if (hidden % 8 || hidden > kMaxPlanesRow || planes < 1 || residual == nullptr) return MSGL_BAD_ARG;
   if (rows == 0) return MSGL_OK;
   if (dtype == MSGL_BF16)
-    return launch_rms_planes<__nv_bfloat16>(x_planes, planes, residual, w, out, out_q, out_scale, rows, hidden, eps,
-                                            plus_one, stream);
+    return launch_rms<__nv_bfloat16>(x_planes, planes, residual, w, out, out_q, out_scale, rows, hidden, eps, plus_one, stream);
   if (dtype == MSGL_F16)
-    return launch_rms_planes<__half>(x_planes, planes, residual, w, out, out_q, out_scale, rows, hidden, eps, plus_one,
-                                     stream);
+    return launch_rms<__half>(x_planes, planes, residual, w, out, out_q, out_scale, rows, hidden, eps, plus_one, stream);
   return MSGL_BAD_ARG;
 }
 
@@ -220,12 +237,12 @@ MSGL_API int msgl_rms_norm_planes(const void* x_planes, int planes, void* residu
 MSGL_API int msgl_rms_norm(const void* x, void* residual, const void* w, void* out, void* out_q,
                            void* out_scale, int rows, int hidden, float eps, int plus_one, int dtype,
                            cudaStream_t stream) {
-  if (hidden % 8 || hidden > 16 * 8 * kRowThreads) return MSGL_BAD_ARG;
+  if (hidden % 8 || hidden > kMaxRow) return MSGL_BAD_ARG;
   if (rows == 0) return MSGL_OK;
   if (dtype == MSGL_BF16)
-    return launch_rms<__nv_bfloat16>(x, residual, w, out, out_q, out_scale, rows, hidden, eps, plus_one, stream);
+    return launch_rms<__nv_bfloat16>(x, 0, residual, w, out, out_q, out_scale, rows, hidden, eps, plus_one, stream);
   if (dtype == MSGL_F16)
-    return launch_rms<__half>(x, residual, w, out, out_q, out_scale, rows, hidden, eps, plus_one, stream);
+    return launch_rms<__half>(x, 0, residual, w, out, out_q, out_scale, rows, hidden, eps, plus_one, stream);
   return MSGL_BAD_ARG;
 }
 
@@ -277,28 +294,43 @@ __global__ void act_mul_kernel(const T* __restrict__ x, T* __restrict__ out, int
   store8(out + row * inter + col, y);
 }
 
-template <typename T, int VPT, int THREADS>
-__global__ void __launch_bounds__(THREADS) act_mul_quant_kernel(const T* __restrict__ x,
-                                                                    uint8_t* __restrict__ out_q,
-                                                                    float* __restrict__ out_scale, int inter,
-                                                                    int kind) {
+// The product is rounded to T before its maximum is taken, so a thread keeps it as T between the two passes. Bound: HBM.
+// KIND is a constant (a branch on it between two vectors' loads made each of up to 14 vectors a memory round trip of
+// its own) and the loads of AHEAD vectors are issued together.
+// B200, us, before -> after: 8192 x 28672 698 -> 310 (3.8 TB/s), 8190 x 9728 86 -> 74.5, 1 x 9728 3.3 -> 2.9.
+template <typename T, int VPT, int THREADS, int KIND>
+__global__ void __launch_bounds__(THREADS) act_mul_quant_kernel(const T* __restrict__ x, uint8_t* __restrict__ out_q,
+                                                                float* __restrict__ out_scale, int inter) {
+  constexpr int AHEAD = VPT < 4 ? VPT : 4;
   pdl_enter();
   __shared__ float scratch[32];
   const int row = blockIdx.x;
   const T* g = x + (size_t)row * 2 * inter;
-  float v[VPT][8];
+  Vec8<T> kept[VPT];
   float amax = 0.f;
 #pragma unroll
-  for (int j = 0; j < VPT; ++j) {
-    const int i = (j * THREADS + threadIdx.x) * 8;
-    if (i < inter) {
-      float a[8], b[8];
-      load8(g + i, a);
-      load8(g + inter + i, b);
+  for (int j0 = 0; j0 < VPT; j0 += AHEAD) {
+    Vec8<T> a[AHEAD], b[AHEAD];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        v[j][k] = to_float(from_float<T>(act_fn(a[k], kind) * b[k]));
-        amax = fmaxf(amax, fabsf(v[j][k]));
+    for (int j = 0; j < AHEAD; ++j) {
+      const int i = ((j0 + j) * THREADS + threadIdx.x) * 8;
+      if (j0 + j < VPT && i < inter) {
+        a[j] = *reinterpret_cast<const Vec8<T>*>(g + i);
+        b[j] = *reinterpret_cast<const Vec8<T>*>(g + inter + i);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < AHEAD; ++j) {
+      const int i = ((j0 + j) * THREADS + threadIdx.x) * 8;
+      if (j0 + j < VPT && i < inter) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float2 ga = to_float2(a[j].v[k]), up = to_float2(b[j].v[k]);
+          const auto y = Pack2<T>::make(act_fn(ga.x, KIND) * up.x, act_fn(ga.y, KIND) * up.y);
+          kept[j0 + j].v[k] = y;
+          const float2 f = to_float2(y);
+          amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
+        }
       }
     }
   }
@@ -308,48 +340,46 @@ __global__ void __launch_bounds__(THREADS) act_mul_quant_kernel(const T* __restr
 #pragma unroll
   for (int j = 0; j < VPT; ++j) {
     const int i = (j * THREADS + threadIdx.x) * 8;
-    if (i < inter) *reinterpret_cast<uint2*>(out_q + (size_t)row * inter + i) = pack8_e4m3(v[j], scale);
+    if (i < inter) {
+      float v[8];
+      unpack8(kept[j], v);
+      *reinterpret_cast<uint2*>(out_q + (size_t)row * inter + i) = pack8_e4m3(v, scale);
+    }
   }
 }
 
-template <typename T>
-static int launch_act_quant(const void* x, void* out_q, void* out_scale, int rows, int inter, int kind,
-                            cudaStream_t s) {
-  // few rows (decode): 512 threads per row keep more loads in flight per row; many rows
-  // (prefill): 128 threads, rows in flight come from the grid
-  const bool wide = rows <= 2048 && inter >= 4096;
-  const int threads = wide ? 512 : kRowThreads;
-  const int vpt = (inter / 8 + threads - 1) / threads;
+template <typename T, int KIND>
+static int launch_act_quant(const void* x, void* out_q, void* out_scale, int rows, int inter, cudaStream_t s) {
+  // the widest block that has a few vectors for every thread; a decode step's few rows take twice the threads, which have
+  // more of a row under way at once
+  const int vecs = inter / 8;
 #define ACT_LAUNCH(V, TH) \
-  msgl_launch(act_mul_quant_kernel<T, V, TH>, dim3(rows), dim3(TH), 0, s, (const T*)x, (uint8_t*)out_q, (float*)out_scale, inter, kind)
-  if (wide) {
-    if (vpt <= 1) ACT_LAUNCH(1, 512);
-    else if (vpt <= 2) ACT_LAUNCH(2, 512);
+  msgl_launch(act_mul_quant_kernel<T, V, TH, KIND>, dim3(rows), dim3(TH), 0, s, (const T*)x, (uint8_t*)out_q, (float*)out_scale, inter)
+  if (vecs > 7 * 512) return MSGL_BAD_ARG;
+  if (vecs > 5 * 256 || (rows <= 2048 && vecs > 512)) {
+    const int vpt = (vecs + 511) / 512;
+    if (vpt <= 2) ACT_LAUNCH(2, 512);
     else if (vpt <= 3) ACT_LAUNCH(3, 512);
     else if (vpt <= 4) ACT_LAUNCH(4, 512);
-    else if (vpt <= 7) ACT_LAUNCH(7, 512);
-    else return MSGL_BAD_ARG;
-    return MSGL_OK;
+    else if (vpt <= 5) ACT_LAUNCH(5, 512);
+    else ACT_LAUNCH(7, 512);
+  } else {
+    const int vpt = (vecs + 255) / 256;
+    if (vecs <= 128) ACT_LAUNCH(1, 128);
+    else if (vpt <= 1) ACT_LAUNCH(1, 256);
+    else if (vpt <= 2) ACT_LAUNCH(2, 256);
+    else if (vpt <= 3) ACT_LAUNCH(3, 256);
+    else ACT_LAUNCH(5, 256);
   }
-  if (inter >= 2048) {
-    // many long rows (prefill): 256 threads per row halve the registers a thread holds between the
-    // two passes, which doubles the resident warps
-    const int v256 = (inter / 8 + 255) / 256;
-    if (v256 <= 1) ACT_LAUNCH(1, 256);
-    else if (v256 <= 2) ACT_LAUNCH(2, 256);
-    else if (v256 <= 3) ACT_LAUNCH(3, 256);
-    else if (v256 <= 5) ACT_LAUNCH(5, 256);
-    else if (v256 <= 8) ACT_LAUNCH(8, 256);
-    else if (v256 <= 14) ACT_LAUNCH(14, 256);
-    else return MSGL_BAD_ARG;
-    return MSGL_OK;
-  }
-  if (vpt <= 1) ACT_LAUNCH(1, kRowThreads);
-  else if (vpt <= 2) ACT_LAUNCH(2, kRowThreads);
-  else if (vpt <= 4) ACT_LAUNCH(4, kRowThreads);
-  else return MSGL_BAD_ARG;
 #undef ACT_LAUNCH
   return MSGL_OK;
+}
+
+template <typename T>
+static int launch_act_quant(const void* x, void* out_q, void* out_scale, int rows, int inter, int kind, cudaStream_t s) {
+  if (kind == ACT_SILU) return launch_act_quant<T, ACT_SILU>(x, out_q, out_scale, rows, inter, s);
+  if (kind == ACT_GELU) return launch_act_quant<T, ACT_GELU>(x, out_q, out_scale, rows, inter, s);
+  return launch_act_quant<T, ACT_GELU_TANH>(x, out_q, out_scale, rows, inter, s);
 }
 
 // alpha, limit: constants of kind 3 (clamped), which has no quantised form
@@ -387,30 +417,90 @@ MSGL_API int msgl_act_and_mul(const void* x, void* out, void* out_q, void* out_s
 // ------------------------------------------------------------------------------------------
 // stand-alone activation quantisers: per token (group == hidden) or per `group` elements
 // ------------------------------------------------------------------------------------------
+// A group is one row of up to 16384 elements (a CTA each, VPT 16-byte vectors a thread, read once), or a run of
+// elements of any multiple of 8 (a power of two of lanes each, vectors 16 bytes a lane). B200, us, a warp for each group of any
+// length and two passes over it -> now: 1 x 4096 3.7 -> 1.8, 256 x 4096 5.1 -> 2.7, 8192 x 8192 53 -> 38; 16640 x 2048 in groups of 128
+// 51 -> 33.
+template <typename T, int VPT>
+__global__ void __launch_bounds__(512) quant_row_kernel(const T* __restrict__ x, uint8_t* __restrict__ out_q,
+                                                        float* __restrict__ out_scale, int group) {
+  pdl_enter();
+  __shared__ float scratch[32];
+  const size_t at = (size_t)blockIdx.x * group;
+  const int step = blockDim.x * 8;
+  Vec8<T> kept[VPT];
+  float amax = 0.f;
+#pragma unroll
+  for (int j = 0; j < VPT; ++j) {
+    const int i = j * step + threadIdx.x * 8;
+    if (i < group) kept[j] = *reinterpret_cast<const Vec8<T>*>(x + at + i);
+  }
+#pragma unroll
+  for (int j = 0; j < VPT; ++j)
+    if (j * step + threadIdx.x * 8 < group) {
+      float v[8];
+      unpack8(kept[j], v);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) amax = fmaxf(amax, fabsf(v[k]));
+    }
+  amax = block_max(amax, scratch);
+  const float scale = fmaxf(amax, 1e-8f) / kFp8Max;
+  if (threadIdx.x == 0) out_scale[blockIdx.x] = scale;
+#pragma unroll
+  for (int j = 0; j < VPT; ++j) {
+    const int i = j * step + threadIdx.x * 8;
+    if (i < group) {
+      float v[8];
+      unpack8(kept[j], v);
+      *reinterpret_cast<uint2*>(out_q + at + i) = pack8_e4m3(v, scale);
+    }
+  }
+}
+
 template <typename T>
 __global__ void quant_group_kernel(const T* __restrict__ x, uint8_t* __restrict__ out_q,
-                                   float* __restrict__ out_scale, int group, size_t total_groups) {
+                                   float* __restrict__ out_scale, int group, int lanes, size_t total_groups) {
   pdl_enter();
-  // one warp per group; groups are contiguous runs of `group` elements (group % 8 == 0)
-  const size_t gidx = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (gidx >= total_groups) return;
-  const int lane = threadIdx.x & 31;
+  const size_t gidx = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / lanes;
+  const bool live = gidx < total_groups;
+  const int lane = threadIdx.x & (lanes - 1);
   const T* src = x + gidx * group;
   float amax = 0.f;
-  for (int i = lane * 8; i < group; i += 256) {
+  for (int i = lane * 8; live && i < group; i += lanes * 8) {
     float v[8];
     load8(src + i, v);
 #pragma unroll
     for (int k = 0; k < 8; ++k) amax = fmaxf(amax, fabsf(v[k]));
   }
-  amax = warp_max(amax);
+  for (int o = lanes >> 1; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  if (!live) return;
   const float scale = fmaxf(amax, 1e-8f) / kFp8Max;
   if (lane == 0) out_scale[gidx] = scale;
-  for (int i = lane * 8; i < group; i += 256) {
+  for (int i = lane * 8; i < group; i += lanes * 8) {
     float v[8];
     load8(src + i, v);
     *reinterpret_cast<uint2*>(out_q + gidx * group + i) = pack8_e4m3(v, scale);
   }
+}
+
+template <typename T>
+static void launch_quant(const void* x, void* out_q, void* out_scale, size_t total, int group, cudaStream_t s) {
+  const int vecs = group / 8;
+  if (vecs > 32 && vecs <= 4 * 512) {
+    const int vpt = vecs <= 64 ? 1 : vecs <= 1024 ? 2 : 4, threads = ((vecs + vpt - 1) / vpt + 31) / 32 * 32;
+#define QUANT_ROW(V) \
+  msgl_launch(quant_row_kernel<T, V>, dim3((unsigned)total), dim3(threads), 0, s, (const T*)x, (uint8_t*)out_q, (float*)out_scale, group)
+    if (vpt == 1) QUANT_ROW(1);
+    else if (vpt == 2) QUANT_ROW(2);
+    else QUANT_ROW(4);
+#undef QUANT_ROW
+    return;
+  }
+  int lanes = 1;
+  while (lanes < vecs && lanes < 32) lanes *= 2;
+  const unsigned blocks = (unsigned)((total * lanes + 255) / 256);
+  msgl_launch(quant_group_kernel<T>, dim3(blocks), dim3(256), 0, s, (const T*)x, (uint8_t*)out_q, (float*)out_scale, group, lanes,
+              total);
 }
 
 MSGL_API int msgl_quant_fp8(const void* x, void* out_q, void* out_scale, int rows, int hidden, int group,
@@ -418,17 +508,10 @@ MSGL_API int msgl_quant_fp8(const void* x, void* out_q, void* out_scale, int row
   if (group <= 0) group = hidden;
   if (hidden % group || group % 8) return MSGL_BAD_ARG;
   if (rows == 0) return MSGL_OK;
-  size_t total = (size_t)rows * (hidden / group);
-  int warps = 8;
-  unsigned blocks = (unsigned)((total + warps - 1) / warps);
-  if (dtype == MSGL_BF16)
-    msgl_launch(quant_group_kernel<__nv_bfloat16>, dim3(blocks), dim3(warps * 32), 0, stream, (const __nv_bfloat16*)x, (uint8_t*)out_q,
-                                                                        (float*)out_scale, group, total);
-  else if (dtype == MSGL_F16)
-    msgl_launch(quant_group_kernel<__half>, dim3(blocks), dim3(warps * 32), 0, stream, (const __half*)x, (uint8_t*)out_q,
-                                                                 (float*)out_scale, group, total);
-  else
-    return MSGL_BAD_ARG;
+  const size_t total = (size_t)rows * (hidden / group);
+  if (dtype == MSGL_BF16) launch_quant<__nv_bfloat16>(x, out_q, out_scale, total, group, stream);
+  else if (dtype == MSGL_F16) launch_quant<__half>(x, out_q, out_scale, total, group, stream);
+  else return MSGL_BAD_ARG;
   MSGL_CHECK_LAUNCH("quant_fp8");
   return MSGL_OK;
 }

@@ -228,6 +228,12 @@ __global__ void __launch_bounds__(128) qk_norm_rope_store_fast_kernel(
 // head, each lane holding eight consecutive elements of the low half and the matching eight of
 // the high half (one 16-byte load each), so a warp covers four heads; the per-head RMS is a
 // reduction over the eight lanes; q leaves as 16-byte stores and fp8 K/V as 8-byte stores.
+//
+// Bound: HBM for a prompt's rows, memory latency for a decode step's. Everything that does not depend on another load (row,
+// position, slot, norm weights, cache scale) is asked for before the first use, so that only the rotation table is a second
+// round trip; asked for where they are used they were five. A cache scale of one, which is what a pool without
+// calibrated scales has, divides nothing.
+// B200, us, 32 query and 8 key heads, fp8 pool: 1 row 3.3 -> 2.1, 2397 rows 16.8 -> 14.5, 8190 rows 51 -> 46.
 template <typename T>
 __global__ void __launch_bounds__(128) qk_norm_rope_store_vec128_kernel(
     const T* __restrict__ qkv, const T* __restrict__ q_w, const T* __restrict__ k_w,
@@ -243,10 +249,30 @@ __global__ void __launch_bounds__(128) qk_norm_rope_store_vec128_kernel(
   const int heads_total = hq + 2 * hk;
   const bool live = head < heads_total;
   const int hd = live ? head : heads_total - 1;          // idle groups shadow the last head (no stores)
+  const bool is_q = hd < hq, is_k = !is_q && hd < hq + hk;
+  const int kvh = is_k ? hd - hq : hd - hq - hk;         // of the heads that are stored
+  int pos = positions[token];
+  const int slot = is_q ? -1 : out_loc[token];
+  const float sc = cache_fp8 && !is_q ? (is_k ? k_scale : v_scale)[kvh] : 1.f;
   const T* src = qkv + (size_t)token * heads_total * D + (size_t)hd * D;
+  const Vec8<T> ra = *reinterpret_cast<const Vec8<T>*>(src + sub * 8), rb = *reinterpret_cast<const Vec8<T>*>(src + H2 + sub * 8);
+  const T* w = is_q ? q_w : is_k ? k_w : nullptr;
+  Vec8<T> rl, rh;
+  if (w != nullptr) {
+    rl = *reinterpret_cast<const Vec8<T>*>(w + sub * 8);
+    rh = *reinterpret_cast<const Vec8<T>*>(w + H2 + sub * 8);
+  }
+  (void)MSGL_OOB(pos, max_pos);
+  pos = pos < 0 ? 0 : (pos >= max_pos ? max_pos - 1 : pos);
+  float4 c0, c1, s0, s1;
+  if (is_q || is_k) {
+    const float4* cs = reinterpret_cast<const float4*>(cos_sin + (size_t)pos * D + sub * 8);
+    const float4* sn = reinterpret_cast<const float4*>(cos_sin + (size_t)pos * D + H2 + sub * 8);
+    c0 = cs[0]; c1 = cs[1]; s0 = sn[0]; s1 = sn[1];
+  }
   float a[8], b[8];
-  load8(src + sub * 8, a);
-  load8(src + H2 + sub * 8, b);
+  unpack8(ra, a);
+  unpack8(rb, b);
   float ss = 0.f;
 #pragma unroll
   for (int t = 0; t < 8; ++t) ss += a[t] * a[t] + b[t] * b[t];
@@ -254,26 +280,18 @@ __global__ void __launch_bounds__(128) qk_norm_rope_store_vec128_kernel(
   ss += __shfl_xor_sync(0xffffffffu, ss, 2);
   ss += __shfl_xor_sync(0xffffffffu, ss, 4);
   if (!live) return;
-  const bool is_q = head < hq, is_k = !is_q && head < hq + hk;
   if (is_q || is_k) {
-    const T* w = is_q ? q_w : k_w;
     if (w != nullptr) {
       const float rstd = rsqrtf(ss / (float)D + eps);
       float wl[8], wh[8];
-      load8(w + sub * 8, wl);
-      load8(w + H2 + sub * 8, wh);
+      unpack8(rl, wl);
+      unpack8(rh, wh);
 #pragma unroll
       for (int t = 0; t < 8; ++t) {
         a[t] = to_float(from_float<T>(a[t] * rstd * wl[t]));
         b[t] = to_float(from_float<T>(b[t] * rstd * wh[t]));
       }
     }
-    int pos = positions[token];
-    (void)MSGL_OOB(pos, max_pos);
-    pos = pos < 0 ? 0 : (pos >= max_pos ? max_pos - 1 : pos);
-    const float4* cs = reinterpret_cast<const float4*>(cos_sin + (size_t)pos * D + sub * 8);
-    const float4* sn = reinterpret_cast<const float4*>(cos_sin + (size_t)pos * D + H2 + sub * 8);
-    const float4 c0 = cs[0], c1 = cs[1], s0 = sn[0], s1 = sn[1];
     const float c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
     const float sv[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
 #pragma unroll
@@ -289,33 +307,28 @@ __global__ void __launch_bounds__(128) qk_norm_rope_store_vec128_kernel(
     store8(dst + H2 + sub * 8, b);
     return;
   }
-  const int kvh = is_k ? head - hq : head - hq - hk;
-  const int slot = out_loc[token];
   if (slot >= 0) (void)MSGL_OOB(slot, num_slots);
   if (slot < 0 || slot >= num_slots) return;
   const int page = slot / page_size, off = slot % page_size;
   const size_t base = (((size_t)page * hk + kvh) * page_size + off) * D;
   void* cache = is_k ? k_cache : v_cache;
   if (cache_fp8) {
-    const float sc = is_k ? k_scale[kvh] : v_scale[kvh];
     uint8_t* dst = (uint8_t*)cache + base;
-    float ra[8], rb[8];
 #pragma unroll
     for (int t = 0; t < 8; ++t) {
-      ra[t] = to_float(from_float<T>(a[t])) / sc;   // same rounding and division as the scalar kernel
-      rb[t] = to_float(from_float<T>(b[t])) / sc;
+      a[t] = to_float(from_float<T>(a[t]));   // same rounding and division as the scalar kernel
+      b[t] = to_float(from_float<T>(b[t]));
     }
-    uint2 pa, pb;
-    pa.x = (uint32_t)float_to_e4m3(ra[0]) | ((uint32_t)float_to_e4m3(ra[1]) << 8) | ((uint32_t)float_to_e4m3(ra[2]) << 16) |
-           ((uint32_t)float_to_e4m3(ra[3]) << 24);
-    pa.y = (uint32_t)float_to_e4m3(ra[4]) | ((uint32_t)float_to_e4m3(ra[5]) << 8) | ((uint32_t)float_to_e4m3(ra[6]) << 16) |
-           ((uint32_t)float_to_e4m3(ra[7]) << 24);
-    pb.x = (uint32_t)float_to_e4m3(rb[0]) | ((uint32_t)float_to_e4m3(rb[1]) << 8) | ((uint32_t)float_to_e4m3(rb[2]) << 16) |
-           ((uint32_t)float_to_e4m3(rb[3]) << 24);
-    pb.y = (uint32_t)float_to_e4m3(rb[4]) | ((uint32_t)float_to_e4m3(rb[5]) << 8) | ((uint32_t)float_to_e4m3(rb[6]) << 16) |
-           ((uint32_t)float_to_e4m3(rb[7]) << 24);
-    *reinterpret_cast<uint2*>(dst + sub * 8) = pa;
-    *reinterpret_cast<uint2*>(dst + H2 + sub * 8) = pb;
+    if (sc != 1.f) {
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        a[t] = a[t] / sc;
+        b[t] = b[t] / sc;
+      }
+    }
+    auto pair = [](const float* v) { return (uint32_t)float2_to_e4m3x2(v[0], v[1]) | ((uint32_t)float2_to_e4m3x2(v[2], v[3]) << 16); };
+    *reinterpret_cast<uint2*>(dst + sub * 8) = make_uint2(pair(a), pair(a + 4));
+    *reinterpret_cast<uint2*>(dst + H2 + sub * 8) = make_uint2(pair(b), pair(b + 4));
   } else {
     T* dst = (T*)cache + base;
     store8(dst + sub * 8, a);
