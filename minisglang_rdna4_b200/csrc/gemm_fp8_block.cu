@@ -249,42 +249,43 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
 
 // ------------------------------------------------------------------------------------------
 // SiLU(gate) * up followed by per-group (128 outputs) e4m3 quantisation: the producer of the second
-// expert GEMM's activations. One warp per (row, group).
+// expert GEMM's activations. Sixteen lanes per (row, group), 16-byte loads. sorted_pair (or null): rows
+// that no (token, expert) pair was given (negative) are left out; of a decode step's rows, which are padded to whole tiles
+// for each expert, that is nearly all of them.
+// B200, us, 768 columns: 16640 rows, 384 of them live, 19.1 -> 8.0; 52096 rows, 35840 live, 59.4 -> 36.9.
 // ------------------------------------------------------------------------------------------
 template <typename T>
-__global__ void silu_mul_quant_group_kernel(const T* __restrict__ x, uint8_t* __restrict__ out_q,
-                                            float* __restrict__ out_scale, int inter, int groups_per_row,
-                                            size_t total_groups) {
+__global__ void __launch_bounds__(256) silu_mul_quant_group_kernel(const T* __restrict__ x, uint8_t* __restrict__ out_q,
+                                                                   float* __restrict__ out_scale,
+                                                                   const int32_t* __restrict__ sorted_pair, int inter,
+                                                                   int groups_per_row, size_t total_groups) {
   pdl_enter();
-  const size_t gidx = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (gidx >= total_groups) return;
-  const int lane = threadIdx.x & 31;
+  const size_t gidx = (size_t)blockIdx.x * (blockDim.x >> 4) + (threadIdx.x >> 4);
   const size_t row = gidx / groups_per_row;
-  const int g0 = (int)(gidx % groups_per_row) * 128;
-  const int i = g0 + lane * 4;
-  const T* gp = x + row * 2 * inter;
-  float v[4] = {0.f, 0.f, 0.f, 0.f};
+  const bool live = gidx < total_groups && (sorted_pair == nullptr || sorted_pair[row] >= 0);
+  const int lane = threadIdx.x & 15;
+  const int i = (int)(gidx % groups_per_row) * 128 + lane * 8;
+  float v[8];
   float amax = 0.f;
-  if (i < inter) {
+  if (live) {
+    float g[8], u[8];
+    load8(x + row * 2 * inter + i, g);
+    load8(x + row * 2 * inter + inter + i, u);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float g = to_float(gp[i + e]), u = to_float(gp[inter + i + e]);
-      const float h = 0.5f * g;
+    for (int e = 0; e < 8; ++e) {
+      const float h = 0.5f * g[e];
       float t;
       asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(h));
-      v[e] = to_float(from_float<T>(fmaf(h, t, h) * u));
+      v[e] = to_float(from_float<T>(fmaf(h, t, h) * u[e]));
       amax = fmaxf(amax, fabsf(v[e]));
     }
   }
-  amax = warp_max(amax);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  if (!live) return;
   const float scale = fmaxf(amax, 1e-8f) / kFp8Max;
   if (lane == 0) out_scale[gidx] = scale;
-  if (i < inter) {
-    const float inv = 1.0f / scale;
-    const uint32_t w = (uint32_t)float2_to_e4m3x2(v[0] * inv, v[1] * inv) |
-                       ((uint32_t)float2_to_e4m3x2(v[2] * inv, v[3] * inv) << 16);
-    *reinterpret_cast<uint32_t*>(out_q + row * inter + i) = w;
-  }
+  *reinterpret_cast<uint2*>(out_q + row * inter + i) = pack8_e4m3(v, scale);
 }
 
 struct MapKey {
@@ -403,22 +404,22 @@ MSGL_API int msgl_gemm_fp8_block_status(int reset) {
   return v;
 }
 
-// x [rows, 2 * inter] (gate columns then up columns) -> e4m3 [rows, inter] + fp32 scales [rows, inter / 128]
-MSGL_API int msgl_silu_mul_quant_group(const void* x, void* out_q, void* out_scale, int rows, int inter, int dtype,
-                                       cudaStream_t stream) {
+// x [rows, 2 * inter] (gate columns then up columns) -> e4m3 [rows, inter] + fp32 scales [rows, inter / 128];
+// sorted_pair [rows] or null: rows with a negative entry are not written
+MSGL_API int msgl_silu_mul_quant_group(const void* x, void* out_q, void* out_scale, const void* sorted_pair, int rows, int inter,
+                                       int dtype, cudaStream_t stream) {
   if (inter % 128 || rows < 0) return MSGL_BAD_ARG;
   if (rows == 0) return MSGL_OK;
   const int gpr = inter / 128;
   const size_t total = (size_t)rows * gpr;
-  const int warps = 8;
-  const unsigned blocks = (unsigned)((total + warps - 1) / warps);
+  const unsigned blocks = (unsigned)((total + 15) / 16);
   cudaError_t e;
   if (dtype == MSGL_BF16)
-    e = msgl_launch(silu_mul_quant_group_kernel<__nv_bfloat16>, dim3(blocks), dim3(warps * 32), 0, stream,
-                    (const __nv_bfloat16*)x, (uint8_t*)out_q, (float*)out_scale, inter, gpr, total);
+    e = msgl_launch(silu_mul_quant_group_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, (const __nv_bfloat16*)x,
+                    (uint8_t*)out_q, (float*)out_scale, (const int32_t*)sorted_pair, inter, gpr, total);
   else if (dtype == MSGL_F16)
-    e = msgl_launch(silu_mul_quant_group_kernel<__half>, dim3(blocks), dim3(warps * 32), 0, stream, (const __half*)x,
-                    (uint8_t*)out_q, (float*)out_scale, inter, gpr, total);
+    e = msgl_launch(silu_mul_quant_group_kernel<__half>, dim3(blocks), dim3(256), 0, stream, (const __half*)x, (uint8_t*)out_q,
+                    (float*)out_scale, (const int32_t*)sorted_pair, inter, gpr, total);
   else
     return MSGL_BAD_ARG;
   if (e != cudaSuccess) { msgl_set_error("silu_mul_quant_group", e); return MSGL_CUDA_ERROR; }

@@ -97,10 +97,13 @@ class MoELayer(BaseOP):
             topk_w, topk_ids = ref.moe_route_grouped(logits, self._k, self._renorm, self._scoring, bias,
                                                      self._routed_scale, self._n_group, self._topk_group)
         elif x.is_cuda and not use_ep and getattr(self, "_tier", None) is None:
-            # the routing kernel also counts the tokens of every local expert for the alignment step
+            # the routing kernel also counts the tokens of every local expert for the alignment step (few pairs are
+            # counted there)
             from ..ops import cuda as K
+            from ..ops.moe_kernels import SMALL_PAIRS
 
-            counts = torch.empty(self._e_local, dtype=torch.int32, device=x.device)
+            if x.shape[0] * self._k > SMALL_PAIRS:
+                counts = torch.empty(self._e_local, dtype=torch.int32, device=x.device)
             topk_w, topk_ids = K.moe_route(logits, self._k, self._renorm, self._scoring, bias, self._routed_scale,
                                            counts, self._e_start, self._e_local)
         else:

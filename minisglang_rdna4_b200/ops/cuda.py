@@ -883,20 +883,22 @@ def gemm_fp8_block(x_q, x_scale, w_q, w_scale, out_dtype=torch.bfloat16, tile_ex
     return out
 
 
-def silu_and_mul_quant_group(x):
+def silu_and_mul_quant_group(x, sorted_pair=None):
     """SiLU(gate) * up of ``x [rows, 2I]`` quantised to e4m3 in groups of 128 outputs:
-    returns ``(q [rows, I], scales [rows, I / 128])``."""
+    returns ``(q [rows, I], scales [rows, I / 128])``. ``sorted_pair [rows]`` (int32): rows with a negative
+    entry are left unwritten."""
     from ._lib import bind, c_i, c_p
 
     if not hasattr(silu_and_mul_quant_group, "_bound"):
-        bind("msgl_silu_mul_quant_group", c_i, [c_p, c_p, c_p, c_i, c_i, c_i, c_p])
+        bind("msgl_silu_mul_quant_group", c_i, [c_p, c_p, c_p, c_p, c_i, c_i, c_i, c_p])
         silu_and_mul_quant_group._bound = True
     assert x.is_contiguous() and x.dim() == 2
     rows, two_i = x.shape
     inter = two_i // 2
     q = torch.empty((rows, inter), dtype=torch.float8_e4m3fn, device=x.device)
     s = torch.empty((rows, inter // 128), dtype=torch.float32, device=x.device)
-    check(lib().msgl_silu_mul_quant_group(_p(x), _p(q), _p(s), rows, inter, _dt(x), _stream()), "silu_mul_quant_group")
+    check(lib().msgl_silu_mul_quant_group(_p(x), _p(q), _p(s), _p(sorted_pair), rows, inter, _dt(x), _stream()),
+          "silu_mul_quant_group")
     _count("silu_and_mul_quant_group", "silu_mul_quant_group_kernel")
     return q, s
 

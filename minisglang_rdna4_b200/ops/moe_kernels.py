@@ -14,11 +14,13 @@ _lib.bind("msgl_moe_route", c_i, [c_p] * 5 + [c_i] * 5 + [c_f, c_i, c_i, c_ll, c
 _lib.bind("msgl_moe_combine32", c_i, [c_p, c_p, c_p, c_p, c_i, c_p, c_ll, c_p, c_i, c_i, c_i, c_i, c_p])
 _lib.bind("msgl_gemm_f32_grouped", c_i, [c_p, c_p, c_p, c_i, c_i, c_i, c_p, c_p])
 _lib.bind("msgl_moe_align", c_i, [c_p, c_p, c_p, c_p, c_p, c_p, c_p, c_p, c_i, c_i, c_i, c_i, c_i, c_i, c_p])
+_lib.bind("msgl_moe_quant_rows", c_i, [c_p] * 4 + [c_i] * 5 + [c_p])
 _lib.bind("msgl_moe_permute", c_i, [c_p, c_p, c_p, c_i, c_i, c_i, c_p, c_i, c_p])
 _lib.bind("msgl_moe_combine", c_i, [c_p, c_p, c_p, c_p, c_i, c_i, c_i, c_i, c_p])
 _lib.bind("msgl_gemm_grouped", c_i, [c_i, c_p, c_ll, c_p, c_p, c_ll, c_i, c_i, c_i, c_p, c_i, c_p, c_p, c_i, c_i, c_p])
 
 BLOCK = 128
+SMALL_PAIRS = 4096      # (token, expert) pairs that the alignment takes in one launch (csrc/moe.cu, kSmallPairs)
 _DT = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
 
 
@@ -54,7 +56,7 @@ def moe_align(topk_ids, e_start: int, e_local: int, counts=None):
     t, k = topk_ids.shape
     dev = topk_ids.device
     rows = max_sorted_rows(t, k, e_local)
-    if counts is None:
+    if counts is None and t * k > SMALL_PAIRS:
         counts = torch.zeros(e_local, dtype=torch.int32, device=dev)
         flat = topk_ids.reshape(-1).long() - e_start
         ok = (flat >= 0) & (flat < e_local)
@@ -71,10 +73,13 @@ def _align_with_counts(topk_ids, counts, e_start, e_local, rows):
     meta = torch.empty(2, dtype=torch.int32, device=dev)
     sorted_pair = torch.empty(rows, dtype=torch.int32, device=dev)
     pair_row = torch.empty(t * k, dtype=torch.int32, device=dev)
-    check(lib().msgl_moe_align(topk_ids.data_ptr(), counts.data_ptr(), offsets.data_ptr(), cursor.data_ptr(),
+    check(lib().msgl_moe_align(topk_ids.data_ptr(), K._p(counts), offsets.data_ptr(), cursor.data_ptr(),
                                tile_expert.data_ptr(), meta.data_ptr(), sorted_pair.data_ptr(), pair_row.data_ptr(),
                                t, k, e_start, e_local, rows, BLOCK, K._stream()), "moe_align")
-    K._count("moe_align", "moe_offsets_kernel+moe_scatter_kernel", 2)
+    if t * k <= SMALL_PAIRS:
+        K._count("moe_align", "moe_align_small_kernel")
+    else:
+        K._count("moe_align", "moe_offsets_kernel+moe_scatter_kernel", 2)
     return sorted_pair, pair_row, tile_expert, meta
 
 
@@ -236,10 +241,24 @@ def quantise_rows(kind: str, xs):
     return K.per_group_quant_fp8(xs, 128)
 
 
-def run_experts_q(kind: str, xq, xsc, tile_expert, weights, out_dtype):
+def quantise_sorted(kind: str, x, pair_row, rows: int, k: int):
+    """``quantise_rows`` of the rows that ``pair_row [T*k]`` sorts by expert, each token quantised once; rows of no pair stay
+    unwritten."""
+    t, h = x.shape
+    per_group = ROW_QUANT[kind] == 2
+    q = torch.empty((rows, h), dtype=torch.float8_e4m3fn, device=x.device)
+    s = torch.empty((rows, h // 128) if per_group else (rows,), dtype=torch.float32, device=x.device)
+    check(lib().msgl_moe_quant_rows(x.data_ptr(), pair_row.data_ptr(), q.data_ptr(), s.data_ptr(), t, h, k,
+                                    128 if per_group else 0, _DT[x.dtype], K._stream()), "moe_quant_rows")
+    K._count("moe_quant_rows", "moe_quant_rows_kernel")
+    return q, s
+
+
+def run_experts_q(kind: str, xq, xsc, tile_expert, weights, out_dtype, sorted_pair=None):
     """The two expert GEMMs with SiLU·mul (+ re-quantisation) between them, on expert-sorted rows
     that are already in the input form of ``kind`` (``quantise_rows``): 16-bit rows for ``bf16``,
-    e4m3 rows with their scales otherwise (python/minisgl/quant/kernels.py:562-873,1181-1331)."""
+    e4m3 rows with their scales otherwise (python/minisgl/quant/kernels.py:562-873,1181-1331). ``sorted_pair``: which rows
+    belong to a pair (the others' results are not defined then)."""
     if kind == "bf16":
         w13, w2 = weights
         return gemm_grouped(K.act_and_mul(gemm_grouped(xq, w13, tile_expert)), w2, tile_expert)
@@ -253,7 +272,7 @@ def run_experts_q(kind: str, xq, xsc, tile_expert, weights, out_dtype):
         return gemm_grouped_w8a8(aq, asc, q2, s2, tile_expert, out_dtype)
     if kind == "fp8_block":
         q13, s13, q2, s2 = weights
-        aq, asc = K.silu_and_mul_quant_group(K.gemm_fp8_block(xq, xsc, q13, s13, out_dtype, tile_expert=tile_expert))
+        aq, asc = K.silu_and_mul_quant_group(K.gemm_fp8_block(xq, xsc, q13, s13, out_dtype, tile_expert=tile_expert), sorted_pair)
         return K.gemm_fp8_block(aq, asc, q2, s2, out_dtype, tile_expert=tile_expert)
     raise ValueError(kind)
 
@@ -265,11 +284,14 @@ def run_experts(kind: str, xs, tile_expert, weights, out_dtype):
 
 
 def moe_forward_quant(kind: str, x, weights, topk_w, topk_ids, expert_offset=0, counts=None):
-    """align → permute → quantise → grouped GEMM → SiLU·mul + quantise → grouped GEMM → combine
+    """align → quantise into sorted rows → grouped GEMM → SiLU·mul + quantise → grouped GEMM → combine
     for quantised expert stacks ``weights`` of ``kind``."""
     e_local = weights[0].shape[0]
     k = topk_ids.shape[1]
     sorted_pair, pair_row, tile_expert, _meta = moe_align(topk_ids, expert_offset, e_local, counts)
-    xs = _permute(x, sorted_pair, k)
-    y = run_experts(kind, xs, tile_expert, weights, x.dtype)
+    if ROW_QUANT[kind] == 0:
+        y = run_experts(kind, _permute(x, sorted_pair, k), tile_expert, weights, x.dtype)
+    else:
+        xq, xsc = quantise_sorted(kind, x, pair_row, sorted_pair.numel(), k)
+        y = run_experts_q(kind, xq, xsc, tile_expert, weights, x.dtype, sorted_pair)
     return _combine(y, topk_w, pair_row, x, k)
