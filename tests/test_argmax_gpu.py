@@ -1,0 +1,29 @@
+"""Arg-max by a cluster of CTAs per row."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _rand(*shape, seed=0, dtype=torch.bfloat16):
+    g = torch.Generator("cuda")
+    g.manual_seed(seed + sum(shape))
+    return torch.randn(*shape, generator=g, device="cuda").to(dtype)
+
+
+@pytest.mark.parametrize("vocab", [1, 5, 2047, 16383, 16384, 16397, 151936])
+@pytest.mark.parametrize("rows", [1, 37, 75, 300])
+def test_argmax_of_shares(vocab, rows):
+    from minisglang_rdna4_b200.ops import cuda as K
+
+    x = _rand(rows, vocab, dtype=torch.float32)
+    top = torch.randint(0, vocab, (rows,), device="cuda")
+    x[torch.arange(rows, device="cuda"), top] = 50.0
+    x[0, :] = 7.0                                        # ties: the first one counts
+    x[-1, vocab - 1] = 100.0                             # the last share's last value
+    assert torch.equal(K.argmax(x).long(), x.argmax(-1))
+    x[0] = float("-inf")
+    assert int(K.argmax(x)[0]) == 0
+    wide = torch.full((rows, vocab + 3), 1000.0, device="cuda")
+    wide[:, :vocab] = x
+    assert torch.equal(K.argmax(wide[:, :vocab]).long(), torch.where(torch.isinf(x.amax(-1)), 0, x.argmax(-1)))
