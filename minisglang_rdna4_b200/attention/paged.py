@@ -45,10 +45,11 @@ class PagedAttentionBackend(BaseAttnBackend):
         self.hq, self.hk, self.d = num_q_heads, num_kv_heads, head_dim
         self.layered = bool(heads)
         self.device = device
-        # The number of KV splits of a decode step depends only on the batch size and the
-        # longest sequence the pool can hold, never on the lengths in the batch: a captured
-        # graph and an eager step then reduce in the same order and agree bit for bit.
-        # ``single_split`` pins it to one (speculative verification must reproduce decode).
+        # The number of KV splits of a decode step, and whether its tiles are dealt to the SMs instead, depend only on
+        # the batch size and the longest sequence the pool can hold; the deal itself depends on the lengths of the
+        # requests, which padding rows do not enter. So a captured graph and an eager step of one size reduce in the same
+        # order and agree bit for bit. ``single_split`` pins it to one split (speculative verification must reproduce
+        # decode).
         self.max_seq_len = max_seq_len
         self.single_split = single_split
         self._workspace: Optional[torch.Tensor] = None
@@ -103,7 +104,7 @@ class PagedAttentionBackend(BaseAttnBackend):
         pool = get_global_ctx().kv_cache
         k_cache, v_cache = pool.k_cache(layer), pool.v_cache(layer)
         extra = dict(window=window, chunk=chunk, softcap=softcap, gate=gate, bias=bias, sink=sink, talk=talk)
-        splits = 1
+        splits, deal = 1, False
         if q.is_cuda:
             from ..ops import cuda as K
 
@@ -118,11 +119,16 @@ class PagedAttentionBackend(BaseAttnBackend):
                     splits = K.talk_splits(md.seq_lens.numel(), q.shape[1], k_cache.shape[1], q.shape[2], reach)
                 else:
                     splits = K.choose_splits(md.seq_lens.numel(), k_cache.shape[1], reach, True)
+                    deal = K.deal_pays(md.seq_lens.numel(), k_cache.shape[1], splits, False)
         return ops.paged_attention(q, k_cache, v_cache, md.block_table, md.cu_q, md.seq_lens, scale, causal=True,
                                    max_q=md.max_q, max_kv=md.max_kv, decode=md.decode,
-                                   workspace=md.workspace if talk is None else self._talk_workspace, splits=splits, **extra)
+                                   workspace=md.workspace if talk is None else self._talk_workspace, splits=splits,
+                                   deal=deal, **extra)
 
-    def forward(self, q, layer: int, batch: Batch, *, scale: float, window: int = 0, swa: bool = False):
+    fuses_quant = True     # ``forward`` takes ``quant``
+
+    def forward(self, q, layer: int, batch: Batch, *, scale: float, window: int = 0, swa: bool = False, quant: bool = False):
+        """``quant``: ``(e4m3 rows, scales)`` where the step's kernels write them on the way."""
         md = batch.attn_metadata
         ctx = get_global_ctx()
         # a sliding-window layer with a pool of its own reads that pool through the step's second block table
@@ -137,11 +143,13 @@ class PagedAttentionBackend(BaseAttnBackend):
                 return K.prefill_attention_tc(
                     q, k_cache, pool.v_cache(layer), block_table, md.prefill_plan, scale,
                     k_scale=pool.k_scale[layer] if fp8 else None, v_scale=pool.v_scale[layer] if fp8 else None)
-        splits = 1
+        splits, deal = 1, False
         if md.decode and not self.single_split and q.is_cuda:
-            from ..ops.cuda import choose_splits
+            from ..ops.cuda import choose_splits, deal_pays
 
-            splits = choose_splits(md.seq_lens.numel(), self.hk, self.max_seq_len or md.max_kv, True)
+            b = md.seq_lens.numel()
+            splits = choose_splits(b, self.hk, self.max_seq_len or md.max_kv, True)
+            deal = deal_pays(b, self.hk, splits, fp8)
         mask = md.mask_swa if (window and md.mask_swa is not None) else md.mask
         return ops.paged_attention(
             q, pool.k_cache(layer), pool.v_cache(layer), block_table, md.cu_q, md.seq_lens, scale,
@@ -149,4 +157,5 @@ class PagedAttentionBackend(BaseAttnBackend):
             k_scale=pool.k_scale[layer] if fp8 else None,
             v_scale=pool.v_scale[layer] if fp8 else None,
             max_q=md.max_q, max_kv=md.max_kv, decode=md.decode, workspace=md.workspace, splits=splits,
+            deal=deal, quant=quant,
         )

@@ -53,6 +53,8 @@ struct AttnArgs {
   float softcap;     // c > 0: scores go through c tanh(s / c)
   const void* gate;  // [rows, Hq * D] logits of a sigmoid on the output (row stride ldg), or null
   long long ldg;
+  int2* shared;      // dealt decode: [B * Hk] first and last worker of a (request, head) that several share, else -1
+  int table_rows;    // requests that its tables in shared memory have room for
 };
 
 __device__ int g_attn_status = 0;
@@ -537,50 +539,103 @@ paged_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArg
   }
 }
 
-// merge split partials: one warp per (query row, head)
-template <typename T, int D>
-__global__ void attn_combine_kernel(const float* __restrict__ ws_o, const float* __restrict__ ws_lse,
-                                    T* __restrict__ out, int rows_heads, int splits,
-                                    const int32_t* __restrict__ cu_q, int B, int hq, const T* __restrict__ gate,
-                                    long long ldg) {
+// Merges the parts of split attention: a CTA per query row, a warp per head, parts in ascending order and the loads of
+// several under way together. Splits: [split][row][head] in the workspace. DEALT: the slots of the workers that share a head; a
+// head of one worker is stored already. out_q (or null): the whole row once more, as e4m3 with one scale, which is
+// what a product with 8-bit rows takes: no kernel of its own then has to read the row again.
+template <typename T, int D, bool DEALT>
+__global__ void __launch_bounds__(D == 256 ? 512 : 1024) attn_combine_kernel(const AttnArgs args, uint8_t* __restrict__ out_q,
+                                                                             float* __restrict__ out_scale) {
   pdl_enter();
-  const int idx = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (idx >= rows_heads) return;
-  const int lane = threadIdx.x & 31;
-  // rows past cu_q[B] belong to no request (padding of a captured batch): the split kernels wrote
-  // no partials for them, so they are zero-filled instead of merged from whatever the workspace holds
-  if (idx >= cu_q[B] * hq) {
-    T* pad = out + (size_t)idx * D + lane * (D / 32);
-#pragma unroll
-    for (int i = 0; i < D / 32; ++i) pad[i] = from_float<T>(0.f);
-    return;
-  }
-  float mx = -INFINITY;
-  for (int s = 0; s < splits; ++s) mx = fmaxf(mx, ws_lse[(size_t)s * rows_heads + idx]);
   constexpr int PER = D / 32;
-  float acc[PER];
-#pragma unroll
-  for (int i = 0; i < PER; ++i) acc[i] = 0.f;
-  float wsum = 0.f;
-  if (mx > -INFINITY) {
-    for (int s = 0; s < splits; ++s) {
-      const float w = exp2f(ws_lse[(size_t)s * rows_heads + idx] - mx);
-      if (w == 0.f) continue;
-      wsum += w;
-      const float* src = ws_o + ((size_t)s * rows_heads + idx) * D + lane * PER;
-#pragma unroll
-      for (int i = 0; i < PER; ++i) acc[i] += w * src[i];
+  constexpr int AHEAD = D == 256 ? 3 : D == 128 ? 6 : 8;   // parts whose loads are under way together
+  __shared__ float scratch[32];
+  const int r = blockIdx.x, lane = threadIdx.x & 31, warps = blockDim.x >> 5, G = args.Hq / args.Hk;
+  if (r >= args.cu_q[args.B] && r < args.total_q) {
+    // a row of no request (padding of a captured batch): nobody wrote parts of it
+    const size_t at = (size_t)r * args.Hq * D;
+    for (int i = threadIdx.x * 8; i < args.Hq * D; i += blockDim.x * 8) {
+      *reinterpret_cast<uint4*>(reinterpret_cast<T*>(args.out) + at + i) = make_uint4(0, 0, 0, 0);
+      if (out_q != nullptr) *reinterpret_cast<uint2*>(out_q + at + i) = make_uint2(0, 0);
     }
+    if (out_q != nullptr && threadIdx.x == 0) out_scale[r] = 1e-8f / kFp8Max;
   }
-  const float inv = wsum > 0.f ? 1.f / wsum : 0.f;
-  T* dst = out + (size_t)idx * D + lane * PER;
-  if (gate != nullptr) {
-    const T* g = gate + (idx / hq) * ldg + (idx % hq) * D + lane * PER;
+  if (DEALT ? r >= args.B : r >= args.cu_q[args.B]) return;
+  const int q_row = DEALT ? args.cu_q[r] : r;
+  float amax = 0.f;
+  for (int head = threadIdx.x >> 5; head < args.Hq; head += warps) {
+    const int2 who = DEALT ? args.shared[r * args.Hk + head / G] : make_int2(0, args.splits - 1);
+    T* const dst = reinterpret_cast<T*>(args.out) + ((size_t)q_row * args.Hq + head) * D + lane * PER;
+    float v[PER];
+    if (who.x >= 0) {
+      const int c0 = who.x, c1 = who.y;
+      auto slot_of = [&](int c) {
+        return DEALT ? (2 * (size_t)c + (c == c0 ? 1 : 0)) * G + head % G : ((size_t)c * args.total_q + q_row) * args.Hq + head;
+      };
+      float mx = -INFINITY, wsum = 0.f;
+      for (int c = c0 + lane; c <= c1; c += 32) mx = fmaxf(mx, args.ws_lse[slot_of(c)]);
+      mx = warp_max(mx);
 #pragma unroll
-    for (int i = 0; i < PER; i += 2) gate2(g + i, acc[i], acc[i + 1]);
+      for (int i = 0; i < PER; ++i) v[i] = 0.f;
+#pragma unroll 1
+      for (int c = c0; c <= c1; c += AHEAD) {
+        float part[AHEAD][PER], lse[AHEAD];
+#pragma unroll
+        for (int p = 0; p < AHEAD; ++p) {
+          lse[p] = -INFINITY;
+          if (c + p > c1) continue;
+          const size_t at = slot_of(c + p);
+          lse[p] = args.ws_lse[at];
+          const float* src = args.ws_o + at * D + lane * PER;
+          if constexpr (PER >= 4) {
+#pragma unroll
+            for (int i = 0; i < PER; i += 4) {
+              const float4 x = *reinterpret_cast<const float4*>(src + i);
+              part[p][i] = x.x; part[p][i + 1] = x.y; part[p][i + 2] = x.z; part[p][i + 3] = x.w;
+            }
+          } else {
+            const float2 x = *reinterpret_cast<const float2*>(src);
+            part[p][0] = x.x; part[p][1] = x.y;
+          }
+        }
+#pragma unroll
+        for (int p = 0; p < AHEAD; ++p) {
+          if (lse[p] == -INFINITY) continue;
+          const float w = exp2f(lse[p] - mx);
+          if (w == 0.f) continue;
+          wsum += w;
+#pragma unroll
+          for (int i = 0; i < PER; ++i) v[i] += w * part[p][i];
+        }
+      }
+      const float inv = wsum > 0.f ? 1.f / wsum : 0.f;
+      if (args.gate != nullptr) {
+        const T* const g = reinterpret_cast<const T*>(args.gate) + q_row * args.ldg + head * D + lane * PER;
+#pragma unroll
+        for (int i = 0; i < PER; i += 2) gate2(g + i, v[i], v[i + 1]);
+      }
+#pragma unroll
+      for (int i = 0; i < PER; ++i) v[i] = to_float(from_float<T>(v[i] * inv));
+#pragma unroll
+      for (int i = 0; i < PER; i += 2) *reinterpret_cast<typename Pack2<T>::type*>(dst + i) = Pack2<T>::make(v[i], v[i + 1]);
+    } else {
+      if (out_q == nullptr) continue;
+#pragma unroll
+      for (int i = 0; i < PER; ++i) v[i] = to_float(dst[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < PER; ++i) amax = fmaxf(amax, fabsf(v[i]));
   }
-#pragma unroll
-  for (int i = 0; i < PER; ++i) dst[i] = from_float<T>(acc[i] * inv);
+  if (out_q == nullptr) return;
+  amax = block_max(amax, scratch);   // (behind its barriers all heads of the row are stored)
+  const float scale = fmaxf(amax, 1e-8f) / kFp8Max;
+  const size_t row_at = (size_t)q_row * args.Hq * D;
+  if (threadIdx.x == 0) out_scale[q_row] = scale;
+  for (int i = threadIdx.x * 8; i < args.Hq * D; i += blockDim.x * 8) {
+    float v[8];
+    load8(reinterpret_cast<const T*>(args.out) + row_at + i, v);
+    *reinterpret_cast<uint2*>(out_q + row_at + i) = pack8_e4m3(v, scale);
+  }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -598,6 +653,167 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {
   return y;
 }
 
+// Running state of one warp's online softmax: O^T, and maximum and sum of heads 2j and 2j + 1 (j = lane & 3)
+template <int D> struct DecodeState {
+  float ot[D / 16][4], m0, m1, l0, l1;
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < D / 16; ++i) ot[i][0] = ot[i][1] = ot[i][2] = ot[i][3] = 0.f;
+    m0 = m1 = -INFINITY;
+    l0 = l1 = 0.f;
+  }
+};
+
+// Q^T fragments (B operand): column n = lane >> 2 is head n of the group; qp: its row (of any head where the group has fewer)
+template <typename T, bool KV8, int D>
+__device__ __forceinline__ void load_query(const T* qp, bool head_ok, uint32_t (&qb)[D / 16][2]) {
+  constexpr bool F16MMA = KV8 || std::is_same<T, __half>::value;
+  constexpr int NMB = D / 16;
+  const int j = threadIdx.x & 3;
+#pragma unroll
+  for (int c = 0; c < NMB; ++c) {
+    float x[4];
+    if (KV8) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[e] = head_ok ? to_float(qp[c * 16 + 4 * j + e]) : 0.f;
+    } else {
+      x[0] = head_ok ? to_float(qp[c * 16 + 2 * j]) : 0.f;
+      x[1] = head_ok ? to_float(qp[c * 16 + 2 * j + 1]) : 0.f;
+      x[2] = head_ok ? to_float(qp[c * 16 + 8 + 2 * j]) : 0.f;
+      x[3] = head_ok ? to_float(qp[c * 16 + 8 + 2 * j + 1]) : 0.f;
+    }
+    qb[c][0] = F16MMA ? pack_f16x2(x[0], x[1]) : pack_bf16x2(x[0], x[1]);
+    qb[c][1] = F16MMA ? pack_f16x2(x[2], x[3]) : pack_bf16x2(x[2], x[3]);
+  }
+}
+
+// TKN tokens from position tok0 on, K and V rows in 128-byte-swizzled planes of PLANE_BYTES at k_s and v_s
+template <typename T, bool KV8, int D, int TKN, int PLANE_BYTES>
+__device__ __forceinline__ void decode_tile(DecodeState<D>& state, const uint32_t (&qb)[D / 16][2], uint32_t k_s, uint32_t v_s, int tok0,
+                                            int kv_lo, int kv_hi, float sm_scale, bool capped, float cap_in, float cap_out) {
+  constexpr bool F16MMA = KV8 || std::is_same<T, __half>::value;
+  constexpr int RB = D * (KV8 ? 1 : 2);
+  constexpr int NMB = D / 16;   // 16-row blocks of O^T
+  const int lane = threadIdx.x & 31, g = lane >> 2, mi = lane >> 3;
+  auto& ot = state.ot;
+  float &m0 = state.m0, &m1 = state.m1, &l0 = state.l0, &l1 = state.l1;
+  // ---- S^T = K Q^T : blocks of 16 tokens x 8 heads
+  float st[TKN / 16][4];
+#pragma unroll
+  for (int tb = 0; tb < TKN / 16; ++tb) {
+    st[tb][0] = st[tb][1] = st[tb][2] = st[tb][3] = 0.f;
+    const int trow = tb * 16 + (mi & 1) * 8 + (lane & 7);
+#pragma unroll
+    for (int cp = 0; cp < RB / 32; ++cp) {
+      const int chunk = 2 * cp + (mi >> 1);
+      uint32_t r[4];
+      ldmatrix_x4(k_s + (chunk >> 3) * PLANE_BYTES + trow * 128 + (((chunk & 7) ^ (trow & 7)) << 4), r);
+      if constexpr (KV8) {
+        // one 16-byte chunk = 16 d = one k-step; the pair of chunks gives two k-steps
+        uint32_t a[4] = {e4m3x2_to_f16x2(r[0]), e4m3x2_to_f16x2(r[1]), e4m3x2_to_f16x2(r[0] >> 16),
+                         e4m3x2_to_f16x2(r[1] >> 16)};
+        mma_16816_f16(st[tb], a, qb[2 * cp][0], qb[2 * cp][1]);
+        uint32_t a2[4] = {e4m3x2_to_f16x2(r[2]), e4m3x2_to_f16x2(r[3]), e4m3x2_to_f16x2(r[2] >> 16),
+                          e4m3x2_to_f16x2(r[3] >> 16)};
+        mma_16816_f16(st[tb], a2, qb[2 * cp + 1][0], qb[2 * cp + 1][1]);
+      } else {
+        // two 16-byte chunks = 16 d = one k-step
+        if (F16MMA) mma_16816_f16(st[tb], r, qb[cp][0], qb[cp][1]);
+        else mma_16816_bf16(st[tb], r, qb[cp][0], qb[cp][1]);
+      }
+    }
+  }
+
+  if (capped) {
+#pragma unroll
+    for (int tb = 0; tb < TKN / 16; ++tb)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) st[tb][e] = cap_score(st[tb][e], cap_in, cap_out);
+  }
+  // ---- scale, mask, online softmax over the token axis (per head column)
+  float mx0 = -INFINITY, mx1 = -INFINITY;
+#pragma unroll
+  for (int tb = 0; tb < TKN / 16; ++tb) {
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) {
+      const int tok = tok0 + tb * 16 + g + 8 * hf;
+      const bool ok = tok >= kv_lo && tok < kv_hi;
+      const float a0 = ok ? st[tb][2 * hf] * sm_scale : -INFINITY;
+      const float a1 = ok ? st[tb][2 * hf + 1] * sm_scale : -INFINITY;
+      st[tb][2 * hf] = a0;
+      st[tb][2 * hf + 1] = a1;
+      mx0 = fmaxf(mx0, a0);
+      mx1 = fmaxf(mx1, a1);
+    }
+  }
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1) {
+    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
+    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
+  }
+  const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);
+  const float ms0 = mn0 == -INFINITY ? 0.f : mn0, ms1 = mn1 == -INFINITY ? 0.f : mn1;
+  const float al0 = fast_exp2(m0 - ms0), al1 = fast_exp2(m1 - ms1);
+  m0 = mn0;
+  m1 = mn1;
+  float sum0 = 0.f, sum1 = 0.f;
+#pragma unroll
+  for (int tb = 0; tb < TKN / 16; ++tb) {
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) {
+      const float p0 = fast_exp2(st[tb][2 * hf] - ms0), p1 = fast_exp2(st[tb][2 * hf + 1] - ms1);
+      st[tb][2 * hf] = p0;
+      st[tb][2 * hf + 1] = p1;
+      sum0 += p0;
+      sum1 += p1;
+    }
+  }
+  l0 = l0 * al0 + sum0;
+  l1 = l1 * al1 + sum1;
+#pragma unroll
+  for (int i = 0; i < NMB; ++i) {
+    ot[i][0] *= al0; ot[i][1] *= al1;
+    ot[i][2] *= al0; ot[i][3] *= al1;
+  }
+
+  // ---- O^T += V^T P^T
+#pragma unroll
+  for (int tb = 0; tb < TKN / 16; ++tb) {
+    uint32_t p01, p23;
+    if (F16MMA) { p01 = pack_f16x2(st[tb][0], st[tb][1]); p23 = pack_f16x2(st[tb][2], st[tb][3]); }
+    else { p01 = pack_bf16x2(st[tb][0], st[tb][1]); p23 = pack_bf16x2(st[tb][2], st[tb][3]); }
+    const uint32_t pb0 = movmatrix_trans(p01), pb1 = movmatrix_trans(p23);
+    if constexpr (KV8) {
+      const int trow = tb * 16 + (mi & 1) * 8 + (lane & 7);
+#pragma unroll
+      for (int cp = 0; cp < D / 32; ++cp) {
+        const int chunk = 2 * cp + (mi >> 1);
+        uint32_t r[4];
+        ldmatrix_x4_trans(v_s + (chunk >> 3) * PLANE_BYTES + trow * 128 + (((chunk & 7) ^ (trow & 7)) << 4), r);
+#pragma unroll
+        for (int c2 = 0; c2 < 2; ++c2) {
+          // rows 0..7 of the block are the even d of the chunk, rows 8..15 the odd d
+          const uint32_t we = __byte_perm(r[2 * c2], r[2 * c2 + 1], 0x6420);
+          const uint32_t wo = __byte_perm(r[2 * c2], r[2 * c2 + 1], 0x7531);
+          uint32_t a[4] = {e4m3x2_to_f16x2(we), e4m3x2_to_f16x2(wo), e4m3x2_to_f16x2(we >> 16),
+                           e4m3x2_to_f16x2(wo >> 16)};
+          mma_16816_f16(ot[2 * cp + c2], a, pb0, pb1);
+        }
+      }
+    } else {
+      const int trow = tb * 16 + (mi >> 1) * 8 + (lane & 7);
+#pragma unroll
+      for (int mb = 0; mb < NMB; ++mb) {
+        const int chunk = 2 * mb + (mi & 1);
+        uint32_t r[4];
+        ldmatrix_x4_trans(v_s + (chunk >> 3) * PLANE_BYTES + trow * 128 + (((chunk & 7) ^ (trow & 7)) << 4), r);
+        if (F16MMA) mma_16816_f16(ot[mb], r, pb0, pb1);
+        else mma_16816_bf16(ot[mb], r, pb0, pb1);
+      }
+    }
+  }
+}
+
 template <typename T, bool KV8, int D, int STAGES, bool EXT>
 __global__ void __launch_bounds__(64)
 paged_decode_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs args) {
@@ -606,13 +822,11 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs a
   // So the step's tables and all older KV may be read at once; only q and the tile that holds
   // position kv_len - 1 wait for pdl_wait().
   constexpr int ESZ = KV8 ? 1 : 2;
-  constexpr int RB = D * ESZ;
-  constexpr int PLANES = RB / 128;
+  constexpr int PLANES = D * ESZ / 128;
   constexpr int PLANE_BYTES = TK * 128;
   constexpr int KV_BYTES = PLANES * PLANE_BYTES;
   constexpr int STAGE_BYTES = 2 * KV_BYTES;
   constexpr int BOX_INNER = 128 / ESZ;
-  constexpr bool F16MMA = KV8 || std::is_same<T, __half>::value;
   constexpr int NMB = D / 16;   // 16-row blocks of O^T
 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -693,38 +907,17 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs a
   // ---------------------------------------------------------------------- consumer warp
   pdl_enter();
   const int j = lane & 3, g = lane >> 2;
-  const int mi = lane >> 3;
   // Q^T fragments (B operand): column n = g is head h*G + g
   uint32_t qb[NMB][2];
-  {
-    const bool head_ok = g < G;
-    const T* qp = reinterpret_cast<const T*>(args.q) + ((size_t)q_row * args.Hq + h * G + (head_ok ? g : 0)) * D;
-#pragma unroll
-    for (int c = 0; c < NMB; ++c) {
-      float x[4];
-      if (KV8) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) x[e] = head_ok ? to_float(qp[c * 16 + 4 * j + e]) : 0.f;
-      } else {
-        x[0] = head_ok ? to_float(qp[c * 16 + 2 * j]) : 0.f;
-        x[1] = head_ok ? to_float(qp[c * 16 + 2 * j + 1]) : 0.f;
-        x[2] = head_ok ? to_float(qp[c * 16 + 8 + 2 * j]) : 0.f;
-        x[3] = head_ok ? to_float(qp[c * 16 + 8 + 2 * j + 1]) : 0.f;
-      }
-      qb[c][0] = F16MMA ? pack_f16x2(x[0], x[1]) : pack_bf16x2(x[0], x[1]);
-      qb[c][1] = F16MMA ? pack_f16x2(x[2], x[3]) : pack_bf16x2(x[2], x[3]);
-    }
-  }
+  load_query<T, KV8, D>(reinterpret_cast<const T*>(args.q) + ((size_t)q_row * args.Hq + h * G + (g < G ? g : 0)) * D, g < G, qb);
   const float k_sc = args.k_scale != nullptr ? args.k_scale[h] : 1.f;
   const float v_sc = args.v_scale != nullptr ? args.v_scale[h] : 1.f;
   const bool capped = EXT && args.softcap > 0.f;
   const float sm_scale = capped ? 1.f : args.scale * k_sc * kLog2e;
   const float cap_in = capped ? 2.f * kLog2e * args.scale * k_sc / args.softcap : 0.f, cap_out = args.softcap * kLog2e;
 
-  float ot[NMB][4];
-#pragma unroll
-  for (int i = 0; i < NMB; ++i) { ot[i][0] = ot[i][1] = ot[i][2] = ot[i][3] = 0.f; }
-  float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;   // heads 2j and 2j+1
+  DecodeState<D> state;
+  state.clear();
 
   int stage = 0;
   uint32_t phase = 0;
@@ -733,127 +926,16 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs a
     const uint32_t k_s = s_base + stage * STAGE_BYTES, v_s = k_s + KV_BYTES;
     const int tok0 = (t_begin + t) * TK;
 
-    // ---- S^T = K Q^T : four blocks of 16 tokens x 8 heads
-    float st[TK / 16][4];
-#pragma unroll
-    for (int tb = 0; tb < TK / 16; ++tb) {
-      st[tb][0] = st[tb][1] = st[tb][2] = st[tb][3] = 0.f;
-      const int trow = tb * 16 + (mi & 1) * 8 + (lane & 7);
-#pragma unroll
-      for (int cp = 0; cp < RB / 32; ++cp) {
-        const int chunk = 2 * cp + (mi >> 1);
-        uint32_t r[4];
-        ldmatrix_x4(k_s + (chunk >> 3) * PLANE_BYTES + trow * 128 + (((chunk & 7) ^ (trow & 7)) << 4), r);
-        if (KV8) {
-          // one 16-byte chunk = 16 d = one k-step; the pair of chunks gives two k-steps
-          uint32_t a[4] = {e4m3x2_to_f16x2(r[0]), e4m3x2_to_f16x2(r[1]), e4m3x2_to_f16x2(r[0] >> 16),
-                           e4m3x2_to_f16x2(r[1] >> 16)};
-          mma_16816_f16(st[tb], a, qb[2 * cp][0], qb[2 * cp][1]);
-          uint32_t a2[4] = {e4m3x2_to_f16x2(r[2]), e4m3x2_to_f16x2(r[3]), e4m3x2_to_f16x2(r[2] >> 16),
-                            e4m3x2_to_f16x2(r[3] >> 16)};
-          mma_16816_f16(st[tb], a2, qb[2 * cp + 1][0], qb[2 * cp + 1][1]);
-        } else {
-          // two 16-byte chunks = 16 d = one k-step
-          if (F16MMA) mma_16816_f16(st[tb], r, qb[cp][0], qb[cp][1]);
-          else mma_16816_bf16(st[tb], r, qb[cp][0], qb[cp][1]);
-        }
-      }
-    }
-
-    if (capped) {
-#pragma unroll
-      for (int tb = 0; tb < TK / 16; ++tb)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) st[tb][e] = cap_score(st[tb][e], cap_in, cap_out);
-    }
-    // ---- scale, mask, online softmax over the token axis (per head column)
-    float mx0 = -INFINITY, mx1 = -INFINITY;
-#pragma unroll
-    for (int tb = 0; tb < TK / 16; ++tb) {
-#pragma unroll
-      for (int hf = 0; hf < 2; ++hf) {
-        const int tok = tok0 + tb * 16 + g + 8 * hf;
-        const bool ok = tok >= kv_lo && tok < kv_hi;
-        const float a0 = ok ? st[tb][2 * hf] * sm_scale : -INFINITY;
-        const float a1 = ok ? st[tb][2 * hf + 1] * sm_scale : -INFINITY;
-        st[tb][2 * hf] = a0;
-        st[tb][2 * hf + 1] = a1;
-        mx0 = fmaxf(mx0, a0);
-        mx1 = fmaxf(mx1, a1);
-      }
-    }
-#pragma unroll
-    for (int o = 4; o < 32; o <<= 1) {
-      mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
-      mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
-    }
-    const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);
-    const float ms0 = mn0 == -INFINITY ? 0.f : mn0, ms1 = mn1 == -INFINITY ? 0.f : mn1;
-    const float al0 = fast_exp2(m0 - ms0), al1 = fast_exp2(m1 - ms1);
-    m0 = mn0;
-    m1 = mn1;
-    float sum0 = 0.f, sum1 = 0.f;
-#pragma unroll
-    for (int tb = 0; tb < TK / 16; ++tb) {
-#pragma unroll
-      for (int hf = 0; hf < 2; ++hf) {
-        const float p0 = fast_exp2(st[tb][2 * hf] - ms0), p1 = fast_exp2(st[tb][2 * hf + 1] - ms1);
-        st[tb][2 * hf] = p0;
-        st[tb][2 * hf + 1] = p1;
-        sum0 += p0;
-        sum1 += p1;
-      }
-    }
-    l0 = l0 * al0 + sum0;
-    l1 = l1 * al1 + sum1;
-#pragma unroll
-    for (int i = 0; i < NMB; ++i) {
-      ot[i][0] *= al0; ot[i][1] *= al1;
-      ot[i][2] *= al0; ot[i][3] *= al1;
-    }
-
-    // ---- O^T += V^T P^T
-#pragma unroll
-    for (int tb = 0; tb < TK / 16; ++tb) {
-      uint32_t p01, p23;
-      if (F16MMA) { p01 = pack_f16x2(st[tb][0], st[tb][1]); p23 = pack_f16x2(st[tb][2], st[tb][3]); }
-      else { p01 = pack_bf16x2(st[tb][0], st[tb][1]); p23 = pack_bf16x2(st[tb][2], st[tb][3]); }
-      const uint32_t pb0 = movmatrix_trans(p01), pb1 = movmatrix_trans(p23);
-      if (KV8) {
-        const int trow = tb * 16 + (mi & 1) * 8 + (lane & 7);
-#pragma unroll
-        for (int cp = 0; cp < D / 32; ++cp) {
-          const int chunk = 2 * cp + (mi >> 1);
-          uint32_t r[4];
-          ldmatrix_x4_trans(v_s + (chunk >> 3) * PLANE_BYTES + trow * 128 + (((chunk & 7) ^ (trow & 7)) << 4), r);
-#pragma unroll
-          for (int c2 = 0; c2 < 2; ++c2) {
-            // rows 0..7 of the block are the even d of the chunk, rows 8..15 the odd d
-            const uint32_t we = __byte_perm(r[2 * c2], r[2 * c2 + 1], 0x6420);
-            const uint32_t wo = __byte_perm(r[2 * c2], r[2 * c2 + 1], 0x7531);
-            uint32_t a[4] = {e4m3x2_to_f16x2(we), e4m3x2_to_f16x2(wo), e4m3x2_to_f16x2(we >> 16),
-                             e4m3x2_to_f16x2(wo >> 16)};
-            mma_16816_f16(ot[2 * cp + c2], a, pb0, pb1);
-          }
-        }
-      } else {
-        const int trow = tb * 16 + (mi >> 1) * 8 + (lane & 7);
-#pragma unroll
-        for (int mb = 0; mb < NMB; ++mb) {
-          const int chunk = 2 * mb + (mi & 1);
-          uint32_t r[4];
-          ldmatrix_x4_trans(v_s + (chunk >> 3) * PLANE_BYTES + trow * 128 + (((chunk & 7) ^ (trow & 7)) << 4), r);
-          if (F16MMA) mma_16816_f16(ot[mb], r, pb0, pb1);
-          else mma_16816_bf16(ot[mb], r, pb0, pb1);
-        }
-      }
-    }
+    decode_tile<T, KV8, D, TK, PLANE_BYTES>(state, qb, k_s, v_s, tok0, kv_lo, kv_hi, sm_scale, capped, cap_in, cap_out);
     __syncwarp();
     if (lane == 0) mbar_arrive(empty_bar(stage));
     if (++stage == STAGES) { stage = 0; phase ^= 1u; }
   }
 
   // ---- finalise: sums over the token lanes, then write heads 2j and 2j+1
+  auto& ot = state.ot;
+  const float m0 = state.m0, m1 = state.m1;
+  float l0 = state.l0, l1 = state.l1;
 #pragma unroll
   for (int o = 4; o < 32; o <<= 1) {
     l0 += __shfl_xor_sync(0xffffffffu, l0, o);
@@ -904,6 +986,351 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs a
       if (ok1) args.ws_lse[(size_t)split * plane + (size_t)q_row * args.Hq + head1] = l1 > 0.f ? m1 + log2f(l1) : -INFINITY;
     }
   }
+}
+
+// ------------------------------------------------------------------------------------------
+// Decode steps, dealt evenly. Every warp is a worker of its own: it keeps two stages of 32 KV tokens, issues the TMA copies of the
+// tile after next itself once it has used a stage up, and has an equal contiguous range of the (request, head, tile) units of the
+// whole step. A part of a (request, head) that other workers share goes to the workspace, and attn_combine_kernel sums the parts.
+//
+// Bound: the dependent ldmatrix -> convert -> mma chains of the warps that fit on an SM (256 requests: 4.9 TB/s, issue slots 40 %
+// busy, 2.8 warps a scheduler). paged_decode_kernel gives a fixed number of splits of each request to a CTA with a producer
+// warp, half of the registers: 6 (fp8) or 3 (16-bit) consuming warps an SM, and the longest request's CTAs run alone in
+// the end. Here all 12 (6) warps consume and finish together. B200, us, with the merge, splits -> dealt: 37 requests of 90 to 3500
+// tokens (fp8) 63.8 -> 49.7, 256 of 512 to 2304 182.5 -> 164.5, 4 of 20000 to 31000 (bf16) 115.3 -> 102.4. Summing the parts by
+// the worker that arrives last took 8 us more: one warp waits for a dozen parts while the rest of the GPU is idle.
+// The deal depends on the lengths of the requests of at least two tiles alone; shorter ones, the padding rows of a captured
+// batch among them, are whole segments and are handed out round robin, so that padding changes nobody's bits.
+// ------------------------------------------------------------------------------------------
+constexpr int DTK = 32;           // KV tokens of a tile
+constexpr int kMostParts = 16;    // parts of a (request, head), about: two rounds of loads of attn_combine_kernel
+constexpr int kDealRows = 1024;   // requests of a call
+
+template <bool EXT> __device__ __forceinline__ int decode_tiles(const AttnArgs& a, int kv_len) {
+  if (kv_len <= 0) return 0;
+  const int lo = first_visible<EXT>(a, kv_len - 1);
+  return kv_len > lo ? (kv_len + DTK - 1) / DTK - lo / DTK : 0;
+}
+
+struct DecodeSegment {
+  int b, h, t_begin, n;   // n tiles of request b, key head h, from tile t_begin on
+  int tiles, first;       // tiles of the whole (request, head), and the unit that it begins at
+};
+
+// Hands out a worker's segments.
+struct DecodeDeal {
+  const int* pre;   // [B + 1] tiles of the requests before, of those that have at least two
+  const int* len;   // [B]
+  int u, u_end, i, step;
+
+  __device__ static int range_of(int units, int worker, int workers) { return (int)((long long)units * worker / workers); }
+  __device__ static int worker_of(int units, int unit, int workers) { return (int)((((long long)unit + 1) * workers - 1) / units); }
+
+  template <bool EXT> __device__ bool next(const AttnArgs& a, DecodeSegment& s) {
+    if (u < u_end) {
+      const int x = u / a.Hk;
+      int lo = 0, hi = a.B;   // the last request that begins at or before x
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (pre[mid] <= x) lo = mid; else hi = mid;
+      }
+      s.b = lo;
+      s.tiles = pre[lo + 1] - pre[lo];
+      const int rem = u - pre[lo] * a.Hk;
+      s.h = rem / s.tiles;
+      const int t0 = rem - s.h * s.tiles;
+      s.n = min(s.tiles - t0, u_end - u);
+      s.first = u - t0;
+      s.t_begin = first_visible<EXT>(a, len[lo] - 1) / DTK + t0;
+      u += s.n;
+      return true;
+    }
+    for (; i < a.B * a.Hk; i += step) {
+      const int b = i / a.Hk;
+      if (pre[b + 1] != pre[b]) continue;
+      s.b = b;
+      s.h = i - b * a.Hk;
+      s.n = s.tiles = decode_tiles<EXT>(a, len[b]);
+      s.first = 0;
+      s.t_begin = s.n > 0 ? first_visible<EXT>(a, len[b] - 1) / DTK : 0;
+      i += step;
+      return true;
+    }
+    return false;
+  }
+};
+
+// warps of a CTA: three CTAs fit on an SM, with 16 KB (32 KB: 16-bit rows of 128) of stages a warp
+template <bool KV8, int D> constexpr int kWorkersOf = !KV8 && D == 128 ? 2 : 4;
+
+template <typename T, bool KV8, int D, bool EXT>
+__global__ void __launch_bounds__(kWorkersOf<KV8, D> * 32, 12 / kWorkersOf<KV8, D>)
+paged_decode_deal_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs args) {
+  // As in paged_decode_kernel, the step's tables and all older KV are read at once; q and the tile with position
+  // kv_len - 1 wait for pdl_wait().
+  constexpr int kWorkers = kWorkersOf<KV8, D>;
+  constexpr int ESZ = KV8 ? 1 : 2;
+  constexpr int PLANES = D * ESZ / 128;
+  constexpr int PLANE_BYTES = DTK * 128;
+  constexpr int KV_BYTES = PLANES * PLANE_BYTES;
+  constexpr int STAGE_BYTES = 2 * KV_BYTES;
+  constexpr int BOX_INNER = 128 / ESZ;
+  constexpr int NMB = D / 16;
+
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t s_base = smem_u32(smem) + warp * 2 * STAGE_BYTES;
+  const uint32_t bars = smem_u32(smem) + kWorkers * 2 * STAGE_BYTES + warp * 16;
+  uint8_t* const after = smem + kWorkers * (2 * STAGE_BYTES + 16);
+  volatile int* const abort_flag = reinterpret_cast<volatile int*>(after) + warp;
+  int* const s_part = reinterpret_cast<int*>(after) + kWorkers;   // [2 * kWorkers]: sums and maxima of the warps
+  int* const len = s_part + 2 * kWorkers;
+  int* const row = len + args.table_rows;
+  int* const pre = row + args.table_rows;
+  const int G = args.Hq / args.Hk;
+  const int ps = args.page_size;
+
+  if (lane == 0) {
+    mbar_init(bars, 1);
+    mbar_init(bars + 8, 1);
+    *abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (threadIdx.x == 0) prefetch_tensormap(&kv_map);
+  int longest = 0;
+  {
+    // lengths, and the tiles before each request: a run of requests per thread, a scan over the threads
+    const int run = (args.B + kWorkers * 32 - 1) / (kWorkers * 32);
+    const int b0 = min((int)threadIdx.x * run, args.B), b1 = min(b0 + run, args.B);
+    int mine = 0;
+#pragma unroll 4
+    for (int b = b0; b < b1; ++b) {
+      const int l = args.seq_lens[b];
+      row[b] = args.cu_q[b];
+      len[b] = l;
+      const int t = decode_tiles<EXT>(args, l);
+      mine += t > 1 ? t : 0;
+      longest = max(longest, t);
+    }
+    int sum = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += up;
+      longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
+    }
+    if (lane == 31) { s_part[warp] = sum; s_part[kWorkers + warp] = longest; }
+    __syncthreads();
+    int before = sum - mine;
+#pragma unroll
+    for (int w = 0; w < kWorkers; ++w) {
+      if (w < warp) before += s_part[w];
+      longest = max(longest, s_part[kWorkers + w]);
+    }
+    for (int b = b0; b < b1; ++b) {
+      pre[b] = before;
+      const int t = decode_tiles<EXT>(args, len[b]);
+      before += t > 1 ? t : 0;
+    }
+    if (threadIdx.x == kWorkers * 32 - 1) pre[args.B] = before;
+    __syncthreads();
+  }
+  const int units = pre[args.B] * args.Hk;
+  const int least = max(1, (longest + kMostParts - 1) / kMostParts);   // tiles that are worth a worker
+  const int workers = max(1, min((int)gridDim.x * kWorkers, units / least));
+  // neighbouring ranges go to different SMs first
+  const int me = warp * gridDim.x + blockIdx.x;
+  DecodeDeal deal{pre, len, 0, 0, me, (int)gridDim.x * kWorkers};
+  if (me < workers) {
+    deal.u = DecodeDeal::range_of(units, me, workers);
+    deal.u_end = DecodeDeal::range_of(units, me + 1, workers);
+  }
+  DecodeDeal ahead = deal;            // of the copies: up to two tiles ahead, across segments
+  DecodeSegment seg, next;
+  bool more = ahead.next<EXT>(args, next), waited = false;
+  int next_t = 0, issued = 0;
+  // lane p has the number of page p of the next tile that is to be copied
+  const int pages_per_tile = DTK / ps;
+  int page = 0;
+  auto ask_page = [&]() {
+    if (more && next.n > 0 && lane < pages_per_tile)
+      page = args.block_table[(size_t)next.b * args.bt_stride + min((next.t_begin + next_t) * pages_per_tile + lane, args.bt_stride - 1)];
+  };
+  auto issue = [&]() {   // the copies of one tile, into the stage that is free
+    while (more && next_t == next.n) {   // segments of no tiles need none
+      more = ahead.next<EXT>(args, next);
+      next_t = 0;
+      ask_page();
+    }
+    if (!more) return;
+    if (!waited && next.t_begin + next_t >= (len[next.b] - 1) / DTK) {
+      pdl_wait();
+      waited = true;
+    }
+    const int stage = issued & 1;
+    const uint32_t k_s = s_base + stage * STAGE_BYTES, v_s = k_s + KV_BYTES, bar = bars + 8 * stage;
+    if (lane == 0) mbar_expect_tx(bar, STAGE_BYTES);
+    __syncwarp();
+    if (lane < pages_per_tile) {
+      int at = page;
+      (void)MSGL_OOB(at, args.num_pages + 1);
+      at = at < 0 ? 0 : (at > args.num_pages ? args.num_pages : at);
+#pragma unroll
+      for (int pl = 0; pl < PLANES; ++pl) {
+        const uint32_t off = pl * PLANE_BYTES + lane * ps * 128;
+        tma_load_5d(k_s + off, &kv_map, bar, pl * BOX_INNER, 0, next.h, at, args.k_coord);
+        tma_load_5d(v_s + off, &kv_map, bar, pl * BOX_INNER, 0, next.h, at, args.v_coord);
+      }
+    }
+    ++issued;
+    if (++next_t == next.n) {
+      more = ahead.next<EXT>(args, next);
+      next_t = 0;
+    }
+    ask_page();
+  };
+  ask_page();
+  issue();
+  issue();
+  pdl_enter();
+
+  const int j = lane & 3, g = lane >> 2;
+  const bool capped = EXT && args.softcap > 0.f;
+  const float cap_out = args.softcap * kLog2e;
+  int used = 0;
+  bool ok = true;
+  while (ok && deal.next<EXT>(args, seg)) {
+    const int b = seg.b, h = seg.h, q_row = row[b], kv_hi = len[b], kv_lo = first_visible<EXT>(args, kv_hi - 1);
+    uint32_t qb[NMB][2];
+    load_query<T, KV8, D>(reinterpret_cast<const T*>(args.q) + ((size_t)q_row * args.Hq + h * G + (g < G ? g : 0)) * D, g < G, qb);
+    const float k_sc = args.k_scale != nullptr ? args.k_scale[h] : 1.f;
+    const float v_sc = args.v_scale != nullptr ? args.v_scale[h] : 1.f;
+    const float sm_scale = capped ? 1.f : args.scale * k_sc * kLog2e;
+    const float cap_in = capped ? 2.f * kLog2e * args.scale * k_sc / args.softcap : 0.f;
+    DecodeState<D> state;
+    state.clear();
+    for (int t = 0; t < seg.n; ++t, ++used) {
+      const int stage = used & 1;
+      if (!mbar_wait(bars + 8 * stage, (used >> 1) & 1, abort_flag, args.status, 213)) *abort_flag = 1;
+      __syncwarp();
+      if (*abort_flag) { ok = false; break; }
+      const uint32_t k_s = s_base + stage * STAGE_BYTES;
+      decode_tile<T, KV8, D, DTK, PLANE_BYTES>(state, qb, k_s, k_s + KV_BYTES, (seg.t_begin + t) * DTK, kv_lo, kv_hi, sm_scale, capped,
+                                               cap_in, cap_out);
+      __syncwarp();
+      issue();
+    }
+    if (!ok) break;
+
+    // ---- sums over the token lanes, then heads 2j and 2j+1
+    auto& ot = state.ot;
+    float l0 = state.l0, l1 = state.l1;
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) {
+      l0 += __shfl_xor_sync(0xffffffffu, l0, o);
+      l1 += __shfl_xor_sync(0xffffffffu, l1, o);
+    }
+    const float inv0 = l0 > 0.f ? v_sc / l0 : 0.f, inv1 = l1 > 0.f ? v_sc / l1 : 0.f;
+    const bool ok0 = 2 * j < G, ok1 = 2 * j + 1 < G;
+    const size_t out_at = ((size_t)q_row * args.Hq + h * G) * D;   // of the group's first head
+    const T* const gate = EXT && args.gate != nullptr ? reinterpret_cast<const T*>(args.gate) + q_row * args.ldg + h * G * D : nullptr;
+    // the two channels of a block that this thread holds of a head: neighbours (fp8), or eight apart
+    auto channel = [&](int c, int hf) { return KV8 ? c * 16 + 2 * g + hf : c * 16 + g + 8 * hf; };
+    if (seg.n == seg.tiles) {
+      if (lane == 0) args.shared[b * args.Hk + h] = make_int2(-1, -1);
+      T* const o0 = reinterpret_cast<T*>(args.out) + out_at + 2 * j * D;
+      T* const o1 = o0 + D;
+      if (EXT && gate != nullptr) {
+        const T* const g0 = gate + (ok0 ? 2 * j * D : 0);
+        const T* const g1 = gate + (ok1 ? (2 * j + 1) * D : 0);
+#pragma unroll
+        for (int c = 0; c < NMB; ++c)
+#pragma unroll
+          for (int hf = 0; hf < 2; ++hf) {
+            ot[c][2 * hf] *= __fdividef(1.f, 1.f + fast_exp2(-kLog2e * to_float(g0[channel(c, hf)])));
+            ot[c][2 * hf + 1] *= __fdividef(1.f, 1.f + fast_exp2(-kLog2e * to_float(g1[channel(c, hf)])));
+          }
+      }
+#pragma unroll
+      for (int c = 0; c < NMB; ++c) {
+        if (KV8) {
+          if (ok0) *reinterpret_cast<typename Pack2<T>::type*>(o0 + channel(c, 0)) = Pack2<T>::make(ot[c][0] * inv0, ot[c][2] * inv0);
+          if (ok1) *reinterpret_cast<typename Pack2<T>::type*>(o1 + channel(c, 0)) = Pack2<T>::make(ot[c][1] * inv1, ot[c][3] * inv1);
+        } else {
+#pragma unroll
+          for (int hf = 0; hf < 2; ++hf) {
+            if (ok0) o0[channel(c, hf)] = from_float<T>(ot[c][2 * hf] * inv0);
+            if (ok1) o1[channel(c, hf)] = from_float<T>(ot[c][2 * hf + 1] * inv1);
+          }
+        }
+      }
+      continue;
+    }
+    // slot [2 * worker + (1: the request begins here)][G]: a worker has at most one of either
+    const int c0 = DecodeDeal::worker_of(units, seg.first, workers), c1 = DecodeDeal::worker_of(units, seg.first + seg.tiles - 1, workers);
+    if (lane == 0 && me == c0) args.shared[b * args.Hk + h] = make_int2(c0, c1);
+    const size_t at = (2 * (size_t)me + (me == c0 ? 1 : 0)) * G + 2 * j;
+    float* const w0 = args.ws_o + at * D;
+    float* const w1 = w0 + D;
+#pragma unroll
+    for (int c = 0; c < NMB; ++c)
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        if (ok0) w0[channel(c, hf)] = ot[c][2 * hf] * inv0;
+        if (ok1) w1[channel(c, hf)] = ot[c][2 * hf + 1] * inv1;
+      }
+    if (g == 0) {
+      if (ok0) args.ws_lse[at] = l0 > 0.f ? state.m0 + log2f(l0) : -INFINITY;
+      if (ok1) args.ws_lse[at + 1] = l1 > 0.f ? state.m1 + log2f(l1) : -INFINITY;
+    }
+  }
+  if (!ok) {   // give copies that are still in flight time to land before the CTA exits
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+  }
+}
+
+// requests that the tables have room for
+int deal_rows(int B) { return B <= 256 ? 256 : B <= 512 ? 512 : kDealRows; }
+
+// CTAs of a dealt call, as many as the GPU holds at once; in *smem their shared memory
+template <typename T, bool KV8, int D, bool EXT = false>
+int deal_ctas(int rows, int* smem) {
+  constexpr int kWorkers = kWorkersOf<KV8, D>;
+  constexpr int fixed = kWorkers * (2 * 2 * (D * (KV8 ? 1 : 2) / 128) * DTK * 128 + 16) + 3 * kWorkers * 4 + 1024;
+  *smem = fixed + (3 * rows + 1) * 4;
+  static int ctas[3] = {0, 0, 0};   // of 256, 512, 1024 table rows
+  const int at = rows == 256 ? 0 : rows == 512 ? 1 : 2;
+  if (ctas[at] == 0) {
+    cudaError_t e = cudaFuncSetAttribute(paged_decode_deal_kernel<T, KV8, D, EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         fixed + (3 * kDealRows + 1) * 4);
+    int per_sm = 0, dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, paged_decode_deal_kernel<T, KV8, D, EXT>, kWorkers * 32, *smem);
+    if (e != cudaSuccess || per_sm <= 0 || sms <= 0) { msgl_set_error("dealt decode attention", e); return -1; }
+    ctas[at] = per_sm * sms;
+  }
+  return ctas[at];
+}
+
+template <typename T, bool KV8, int D, bool EXT = false>
+int launch_deal(const CUtensorMap& map, const AttnArgs& a, void* out_q, void* out_scale, cudaStream_t stream) {
+  constexpr int kWorkers = kWorkersOf<KV8, D>;
+  int smem = 0;
+  int ctas = deal_ctas<T, KV8, D, EXT>(a.table_rows, &smem);
+  if (ctas < 0) return MSGL_CUDA_ERROR;
+  // never more warps than there can be tiles (which leaves the deal as it is)
+  const long long most = (long long)a.B * a.Hk * (((long long)a.bt_stride * a.page_size + DTK - 1) / DTK);
+  if (most < (long long)ctas * kWorkers) ctas = (int)((most + kWorkers - 1) / kWorkers);
+  if (ctas < 1) ctas = 1;
+  msgl_launch(paged_decode_deal_kernel<T, KV8, D, EXT>, dim3(ctas), dim3(kWorkers * 32), smem, stream, map, a);
+  msgl_launch(attn_combine_kernel<T, D, true>, dim3(a.total_q > a.B ? a.total_q : a.B), dim3(a.Hq < 32 ? a.Hq * 32 : 1024), 0, stream,
+              a, (uint8_t*)out_q, (float*)out_scale);
+  MSGL_CHECK_LAUNCH("paged_decode_deal");
+  return MSGL_OK;
 }
 
 template <typename T, bool KV8, int D, int STAGES, bool EXT = false>
@@ -1035,18 +1462,38 @@ MSGL_API int msgl_attn_make_kv_map(void* out_map, const void* pool, int elem_byt
   return MSGL_OK;
 }
 
+// Whether msgl_paged_decode covers a call: the workers that share it out (of [2 * workers * hq / hk * (head_dim + 1)] floats of
+// workspace), or 0.
+MSGL_API int msgl_paged_decode_workers(int B, int hq, int hk, int head_dim, int page_size, int kv_fp8, int ext, int dtype) {
+  if (g_force_general_decode || B <= 0 || B > kDealRows || hk <= 0 || hq % hk || hq / hk > 8) return 0;
+  if (page_size < 8 || DTK % page_size) return 0;
+  if (ext && (kv_fp8 || dtype != MSGL_BF16)) return 0;
+  const int rows = deal_rows(B);
+  int smem = 0, ctas = 0;
+  if (ext) ctas = head_dim == 128 ? deal_ctas<__nv_bfloat16, false, 128, true>(rows, &smem)
+                  : head_dim == 64 ? deal_ctas<__nv_bfloat16, false, 64, true>(rows, &smem) : 0;
+  else if (dtype == MSGL_BF16) ctas = head_dim == 128 ? (kv_fp8 ? deal_ctas<__nv_bfloat16, true, 128>(rows, &smem)
+                                                                : deal_ctas<__nv_bfloat16, false, 128>(rows, &smem))
+                                      : head_dim == 64 && !kv_fp8 ? deal_ctas<__nv_bfloat16, false, 64>(rows, &smem) : 0;
+  else if (dtype == MSGL_F16) ctas = head_dim == 128 ? (kv_fp8 ? deal_ctas<__half, true, 128>(rows, &smem)
+                                                               : deal_ctas<__half, false, 128>(rows, &smem))
+                                     : head_dim == 64 && !kv_fp8 ? deal_ctas<__half, false, 64>(rows, &smem) : 0;
+  return ctas > 0 ? ctas * (!kv_fp8 && head_dim == 128 ? kWorkersOf<false, 128> : kWorkersOf<true, 128>) : 0;
+}
+
 // Workspace sizes (floats) for `splits` partials of `total_q` rows.
 MSGL_API long long msgl_attn_workspace_floats(int total_q, int hq, int head_dim, int splits) {
   return (long long)splits * total_q * hq * (head_dim + 1);
 }
 
+// out_q, out_scale (or null; splits > 1): the output rows as e4m3 [total_q, hq * head_dim] with a scale each
 MSGL_API int msgl_paged_attention(const void* kv_map, const void* q, void* out, const void* block_table,
                                   int bt_stride, const void* cu_q, const void* seq_lens, const void* k_scale,
                                   const void* v_scale, const void* mask, long long mask_stride, void* workspace,
                                   int B, int total_q, int max_q, int hq, int hk, int head_dim, int page_size,
                                   int num_pages, int layer, int num_layers, int kv_fp8, int causal, int window,
                                   int splits, float scale, int chunk, float softcap, const void* gate,
-                                  long long ldg, int dtype, cudaStream_t stream) {
+                                  long long ldg, void* out_q, void* out_scale, int dtype, cudaStream_t stream) {
   if (B == 0 || total_q == 0) return MSGL_OK;
   if (hq % hk || hq / hk > 64) {
     msgl_set_error_text("attention: up to 64 query heads per key / value head");
@@ -1058,7 +1505,8 @@ MSGL_API int msgl_paged_attention(const void* kv_map, const void* q, void* out, 
     return MSGL_BAD_ARG;
   }
   if (splits < 1) splits = 1;
-  if (splits > 1 && workspace == nullptr) return MSGL_BAD_ARG;
+  if (splits > 1 && (workspace == nullptr || (uintptr_t)workspace % 16)) return MSGL_BAD_ARG;
+  if (out_q != nullptr && (splits == 1 || out_scale == nullptr)) return MSGL_BAD_ARG;
   AttnArgs a;
   a.q = q; a.out = out;
   a.block_table = (const int32_t*)block_table; a.bt_stride = bt_stride;
@@ -1078,6 +1526,8 @@ MSGL_API int msgl_paged_attention(const void* kv_map, const void* q, void* out, 
   int* status = nullptr;
   cudaGetSymbolAddress((void**)&status, g_attn_status);
   a.status = status;
+  a.shared = nullptr;
+  a.table_rows = 0;
   const CUtensorMap& map = *reinterpret_cast<const CUtensorMap*>(kv_map);
   int rc;
   if (ext) rc = dispatch_attn_ext<__nv_bfloat16>(map, a, head_dim, max_q, stream);
@@ -1086,10 +1536,10 @@ MSGL_API int msgl_paged_attention(const void* kv_map, const void* q, void* out, 
   else return MSGL_BAD_ARG;
   if (rc) return rc;
   if (splits > 1) {
-    const int rows_heads = total_q * hq;
-    const int warps = 4;
-    const int blocks = (rows_heads + warps - 1) / warps;
-#define COMBINE(T, D) msgl_launch(attn_combine_kernel<T, D>, dim3(blocks), dim3(warps * 32), 0, stream, a.ws_o, a.ws_lse, (T*)out, rows_heads, splits, a.cu_q, a.B, a.Hq, (const T*)a.gate, a.ldg)
+    const int most = head_dim == 256 ? 16 : 32;   // warps
+#define COMBINE(T, D)                                                                                                             \
+  msgl_launch(attn_combine_kernel<T, D, false>, dim3(total_q), dim3((hq < most ? hq : most) * 32), 0, stream, a, (uint8_t*)out_q, \
+              (float*)out_scale)
     if (dtype == MSGL_BF16) {
       if (head_dim == 128) COMBINE(__nv_bfloat16, 128);
       else if (head_dim == 256) COMBINE(__nv_bfloat16, 256);
@@ -1103,6 +1553,51 @@ MSGL_API int msgl_paged_attention(const void* kv_map, const void* q, void* out, 
     MSGL_CHECK_LAUNCH("attn_combine");
   }
   return MSGL_OK;
+}
+
+// One query row per request, tiles dealt evenly (paged_decode_deal_kernel). ws: fp32, as msgl_paged_decode_workers says, and
+// 2 * B * hk + 2 words more. out_q, out_scale (or null): the rows as e4m3 [total_q, hq * head_dim] with a scale each.
+MSGL_API int msgl_paged_decode(const void* kv_map, const void* q, void* out, const void* block_table, int bt_stride,
+                               const void* cu_q, const void* seq_lens, const void* k_scale, const void* v_scale, void* ws,
+                               void* out_q, void* out_scale, int B, int total_q, int hq, int hk, int head_dim, int page_size,
+                               int num_pages, int layer, int num_layers, int kv_fp8, int window, float scale, int chunk,
+                               float softcap, const void* gate, long long ldg, int dtype, cudaStream_t stream) {
+  if (B == 0 || total_q == 0) return MSGL_OK;
+  const bool ext = chunk > 0 || softcap > 0.f || gate != nullptr;
+  const int workers = msgl_paged_decode_workers(B, hq, hk, head_dim, page_size, kv_fp8, ext ? 1 : 0, dtype);
+  if (workers == 0 || ws == nullptr || (uintptr_t)ws % 16 || (uintptr_t)out % 16 || (out_q != nullptr && out_scale == nullptr)) {
+    msgl_set_error_text("paged_decode: call not covered");
+    return MSGL_BAD_ARG;
+  }
+  AttnArgs a = {};
+  a.q = q; a.out = out;
+  a.block_table = (const int32_t*)block_table; a.bt_stride = bt_stride;
+  a.cu_q = (const int32_t*)cu_q; a.seq_lens = (const int32_t*)seq_lens;
+  a.k_scale = (const float*)k_scale; a.v_scale = (const float*)v_scale;
+  a.ws_o = (float*)ws;
+  a.ws_lse = a.ws_o + (size_t)2 * workers * (hq / hk) * head_dim;
+  a.shared = reinterpret_cast<int2*>(a.ws_lse + (size_t)2 * workers * (hq / hk));
+  a.B = B; a.Hq = hq; a.Hk = hk; a.page_size = page_size; a.num_pages = num_pages;
+  a.k_coord = layer; a.v_coord = num_layers + layer;
+  a.causal = 1; a.window = window; a.splits = 1; a.total_q = total_q;
+  a.scale = scale;
+  a.chunk = chunk; a.softcap = softcap; a.gate = gate; a.ldg = ldg;
+  a.table_rows = deal_rows(B);
+  int* status = nullptr;
+  cudaGetSymbolAddress((void**)&status, g_attn_status);
+  a.status = status;
+  const CUtensorMap& map = *reinterpret_cast<const CUtensorMap*>(kv_map);
+  using bf16 = __nv_bfloat16;
+  if (ext) return head_dim == 128 ? launch_deal<bf16, false, 128, true>(map, a, out_q, out_scale, stream)
+                                  : launch_deal<bf16, false, 64, true>(map, a, out_q, out_scale, stream);
+  if (dtype == MSGL_BF16) {
+    if (head_dim == 64) return launch_deal<bf16, false, 64>(map, a, out_q, out_scale, stream);
+    return kv_fp8 ? launch_deal<bf16, true, 128>(map, a, out_q, out_scale, stream)
+                  : launch_deal<bf16, false, 128>(map, a, out_q, out_scale, stream);
+  }
+  if (head_dim == 64) return launch_deal<__half, false, 64>(map, a, out_q, out_scale, stream);
+  return kv_fp8 ? launch_deal<__half, true, 128>(map, a, out_q, out_scale, stream)
+                : launch_deal<__half, false, 128>(map, a, out_q, out_scale, stream);
 }
 
 // Test hook: route decode batches through the general (prefill/verify) kernel.
@@ -1173,5 +1668,5 @@ int msgl_paged_attention_noalloc(const void* kv_map, const void* q, void* out, c
   }
   return msgl_paged_attention(kv_map, q, out, block_table, bt_stride, cu_q, seq_lens, k_scale, v_scale, mask,
                               mask_stride, ws, B, total_q, max_q, hq, hk, head_dim, page_size, num_pages, layer,
-                              num_layers, kv_fp8, causal, window, splits, scale, 0, 0.f, nullptr, 0, dtype, stream);
+                              num_layers, kv_fp8, causal, window, splits, scale, 0, 0.f, nullptr, 0, nullptr, nullptr, dtype, stream);
 }

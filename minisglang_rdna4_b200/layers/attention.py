@@ -9,6 +9,7 @@ import torch
 from .. import ops
 from ..core import get_global_ctx
 from ..models.config import RotaryConfig
+from ..quant.method import ActQ, LinearInput
 from .base import BaseOP
 from .rotary import get_rope_cache
 
@@ -36,7 +37,9 @@ class AttentionLayer(BaseOP):
         self._kv_donor: Optional[int] = None
 
     def forward(self, qkv: torch.Tensor, q_norm_w: Optional[torch.Tensor] = None,
-                k_norm_w: Optional[torch.Tensor] = None) -> torch.Tensor:
+                k_norm_w: Optional[torch.Tensor] = None, quant: bool = False) -> LinearInput:
+        """``quant``: the rows go into a product that takes them in 8 bits; they come as an ``ActQ`` where the attention
+        kernels write them so on the way."""
         ctx = get_global_ctx()
         batch = ctx.batch
         if self._cos_sin is None:
@@ -59,5 +62,8 @@ class AttentionLayer(BaseOP):
         )
         if getattr(pool, "amax", None) is not None:
             pool.observe_written(layer, out_loc)
-        out = ctx.attn_backend.forward(q, layer, batch, scale=self._scale, window=self._window, swa=self._swa)
+        extra = {"quant": True} if quant and getattr(ctx.attn_backend, "fuses_quant", False) else {}
+        out = ctx.attn_backend.forward(q, layer, batch, scale=self._scale, window=self._window, swa=self._swa, **extra)
+        if isinstance(out, tuple):
+            return ActQ(*out)
         return out.reshape(out.shape[0], self._hq * self._d)

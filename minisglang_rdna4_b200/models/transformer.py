@@ -62,9 +62,9 @@ class SelfAttention(BaseOP):
     def forward(self, x):
         qkv = self.qkv_proj.forward(x)
         if self._qk_norm:
-            o = self.attn.forward(qkv, self.q_norm.weight, self.k_norm.weight)
+            o = self.attn.forward(qkv, self.q_norm.weight, self.k_norm.weight, quant=self.o_proj.wants_act_quant)
         else:
-            o = self.attn.forward(qkv)
+            o = self.attn.forward(qkv, quant=self.o_proj.wants_act_quant)
         return self.o_proj.forward(o)  # partial sum
 
 

@@ -65,7 +65,7 @@ _SIGNATURES = {
     "msgl_attn_workspace_floats": (c_ll, [c_i, c_i, c_i, c_i]),
     "msgl_paged_attention": (c_i, [c_p, c_p, c_p, c_p, c_i, c_p, c_p, c_p, c_p, c_p, c_ll, c_p,
                                    c_i, c_i, c_i, c_i, c_i, c_i, c_i, c_i, c_i, c_i, c_i, c_i, c_i, c_i,
-                                   c_f, c_i, c_f, c_p, c_ll, c_i, c_p]),
+                                   c_f, c_i, c_f, c_p, c_ll, c_p, c_p, c_i, c_p]),
     "msgl_paged_attention_f32": (c_i, [c_p] * 5 + [c_i, c_p, c_p] + [c_i] * 9 + [c_f, c_f, c_p, c_ll, c_p, c_i, c_p, c_i, c_i,
                                                                               c_p]),
     "msgl_talk_attention": (c_i, [c_p] * 5 + [c_i] + [c_p] * 3 + [c_i] + [c_p] * 3 + [c_i] * 10 + [c_f, c_p]),
@@ -79,6 +79,8 @@ _SIGNATURES = {
                                    c_p, c_p, c_i, c_i, c_i, c_i, c_i, c_i, c_f, c_i, c_i, c_f, c_p, c_ll, c_p, c_i, c_i, c_p, c_i,
                                    c_i, c_i, c_p]),
     "msgl_attn_tc_status": (c_i, [c_i]),
+    "msgl_paged_decode_workers": (c_i, [c_i] * 8),
+    "msgl_paged_decode": (c_i, [c_p] * 4 + [c_i] + [c_p] * 7 + [c_i] * 11 + [c_f, c_i, c_f, c_p, c_ll, c_i, c_p]),
     "msgl_attn_force_general_decode": (None, [c_i]),
     "msgl_attn_decode_stages": (None, [c_i]),
     "msgl_argmax": (c_i, [c_p, c_p, c_i, c_i, c_ll, c_p]),

@@ -291,7 +291,26 @@ def make_pool_buffer(num_layers, pages_plus_one, hk, page_size, d, dtype, device
 
 
 def attention_workspace(max_rows, hq, d, device, max_splits=16):
-    return workspace("attention split partials", max_splits * max_rows * hq * (d + 1), torch.float32, device)
+    """Partials of split attention: every split of every row, or two parts of (up to 8) heads for every worker of a dealt decode
+    step (up to 16 on an SM)."""
+    dealt = 2 * 16 * torch.cuda.get_device_properties(device).multi_processor_count * min(hq, 8) * (d + 1) + 2 * max_rows * hq + 2
+    return workspace("attention split partials", max(max_splits * max_rows * hq * (d + 1), dealt), torch.float32, device)
+
+
+def _row8(q):
+    t, hq, d = q.shape
+    return (torch.empty((t, hq * d), dtype=torch.float8_e4m3fn, device=q.device),
+            torch.empty((t,), dtype=torch.float32, device=q.device))
+
+
+def deal_pays(batch, hk, splits, fp8):
+    """Whether a decode step's tiles are better dealt out by the lengths (``paged_decode_deal_kernel``) than cut into ``splits``
+    for each request. B200, us, cut -> dealt: few requests have few tiles, and the deal's tables cost more than it evens
+    out (fp8, 8 key heads: 1 x 700 tokens 15.1 -> 19.2, 8 x 300 15.9 -> 18.9, 16 x 4000 45.7 -> 48.3); with 32 equal ones it
+    costs 5 (51.3 -> 56.7), with unequal ones it gains three times that (37 x 90 to 3500 63.8 -> 49.7, 256 x 512 to 2304
+    182.5 -> 164.5). Few long ones: where the splits need a second wave (4 x 20000 to 31000 bf16, 512 CTAs of which 444 fit,
+    115.3 -> 102.4)."""
+    return batch * hk >= 192 or batch * hk * splits > (888 if fp8 else 444)
 
 
 def choose_splits(batch, hk, max_kv, decode):
@@ -305,8 +324,11 @@ def choose_splits(batch, hk, max_kv, decode):
 
 def paged_attention(q, k_cache, v_cache, block_table, cu_q, seq_lens, scale, *, causal=True, window=0, mask=None,
                     k_scale=None, v_scale=None, max_q=0, max_kv=0, decode=False, workspace=None, splits=None,
-                    plan=None, tc=None, mask_window=0, chunk=0, softcap=0.0, gate=None, bias=None, sink=None, talk=None):
-    """``plan`` (a ``PrefillPlan``) or ``tc=True`` sends a causal prefill / extend step to the
+                    plan=None, tc=None, mask_window=0, chunk=0, softcap=0.0, gate=None, bias=None, sink=None, talk=None,
+                    deal=False, quant=False):
+    """``quant``: where the kernel that writes the output can, ``(e4m3 rows [T, H * width], a scale per row)`` in its
+    place. ``deal``: a decode step's tiles are shared out evenly over the SMs whatever ``splits`` says
+    (``paged_decode_deal_kernel``), where that form covers the shape. ``plan`` (a ``PrefillPlan``) or ``tc=True`` sends a causal prefill / extend step to the
     tcgen05 kernel when it covers the shape (``tc=True`` without a plan builds the step tables from
     the device lengths, which synchronises). Without either the general kernel runs: decode and
     verification steps must not change kernels with the number of rows per request."""
@@ -336,6 +358,22 @@ def paged_attention(q, k_cache, v_cache, block_table, cu_q, seq_lens, scale, *, 
         max_q = int((cu_q[1:] - cu_q[:-1]).max())
     if max_kv <= 0:
         max_kv = int(seq_lens.max())
+    fp8 = k_cache.dtype == torch.float8_e4m3fn
+    if deal and max_q == 1 and mask is None and causal:
+        ext = chunk > 0 or softcap > 0 or gate is not None
+        workers = int(lib().msgl_paged_decode_workers(b, hq, hk, d, ps, int(fp8), int(ext), _dt(q)))
+        if workers > 0:
+            need = 2 * workers * (hq // hk) * (d + 1) + 2 * b * hk + 2
+            if workspace is None or workspace.numel() < need:
+                workspace = torch.empty(need, dtype=torch.float32, device=q.device)
+            out = torch.empty_like(q)
+            out_q, out_s = _row8(q) if quant else (None, None)
+            check(lib().msgl_paged_decode(
+                desc.ctypes.data, _p(q), _p(out), _p(block_table), block_table.stride(0), _p(cu_q), _p(seq_lens), _p(k_scale),
+                _p(v_scale), _p(workspace), _p(out_q), _p(out_s), b, t, hq, hk, d, ps, pages_p1 - 1, layer, layers, int(fp8),
+                int(window), float(scale), int(chunk), float(softcap), *_output_gate(gate, q), _dt(q), _stream()), "paged_decode")
+            _count("paged_attention", "paged_decode_deal_kernel", 2)
+            return (out_q, out_s) if quant else out
     if splits is None:
         splits = choose_splits(b, hk, max_kv, decode or max_q == 1)
     if splits > 1:
@@ -343,7 +381,7 @@ def paged_attention(q, k_cache, v_cache, block_table, cu_q, seq_lens, scale, *, 
         if workspace is None or workspace.numel() < need:
             workspace = torch.empty(need, dtype=torch.float32, device=q.device)
     out = torch.empty_like(q)
-    fp8 = k_cache.dtype == torch.float8_e4m3fn
+    out_q, out_s = _row8(q) if quant and splits > 1 else (None, None)
     mask_stride = 0
     if mask is not None:
         assert mask.dtype == torch.float32 and mask.stride(-1) == 1
@@ -357,9 +395,9 @@ def paged_attention(q, k_cache, v_cache, block_table, cu_q, seq_lens, scale, *, 
         desc.ctypes.data, _p(q), _p(out), _p(block_table), block_table.stride(0), _p(cu_q), _p(seq_lens),
         _p(k_scale), _p(v_scale), _p(mask), mask_stride, _p(workspace) if splits > 1 else None,
         b, t, max_q, hq, hk, d, ps, pages_p1 - 1, layer, layers, int(fp8), int(causal), int(window), splits,
-        float(scale), int(chunk), float(softcap), *_output_gate(gate, q), _dt(q), _stream()), "paged_attention")
+        float(scale), int(chunk), float(softcap), *_output_gate(gate, q), _p(out_q), _p(out_s), _dt(q), _stream()), "paged_attention")
     _count("paged_attention", "paged_attention_kernel", 2 if splits > 1 else 1)
-    return out
+    return out if out_q is None else (out_q, out_s)
 
 
 def _output_gate(gate, q):
