@@ -288,6 +288,262 @@ __global__ void __launch_bounds__(256) silu_mul_quant_group_kernel(const T* __re
   *reinterpret_cast<uint2*>(out_q + row * inter + i) = pack8_e4m3(v, scale);
 }
 
+// ------------------------------------------------------------------------------------------
+// Grouped form for few rows per expert (decode steps): the product is a read of the experts' weights.
+//
+// Bound: HBM bytes of the weights. The kernel above stages 128 rows of tokens, nearly all of them padding, beside every 128 weight
+// rows, which leaves half of the ring to weights, and its promotion is 128 columns wide. Here the weights are the 128-row side
+// of the MMA and an expert's rows come in tiles of NB = 16 or 32, the columns: 12 or 10 stages of weights are
+// in flight, and a thread promotes the NB columns of its weight row. Every K block is still promoted on its own with
+// the product of its two scales, in ascending order: the same sums. GLU: a work item is 128 gate rows and
+// the 128 up rows that belong to them, so SiLU(gate) * up, and its maximum over the group of 128 outputs, are at hand in the
+// registers of one warpgroup, and e4m3 rows leave the kernel in the place of 16-bit ones that a kernel of its own read again.
+// B200, us of a whole expert layer (8 of 128 experts, 2048 columns, 768 wide; the weights alone take 92), 128-row tiles -> this:
+// 1 token 31.7 -> 34.3, 4: 66.6 -> 61.4, 16: 157 -> 109, 48: 203 -> 135, 128: 211 -> 151, 256 (NB 32): 224 -> 182, 320: 222 -> 184. Tiles of
+// 64 rows took 280.
+// ------------------------------------------------------------------------------------------
+constexpr int kFewBlocks = 32;     // K blocks, at most
+
+template <int NB> struct FewCfg {
+  static constexpr int X_BYTES = NB * BK;
+  static constexpr int SCALE_BYTES = NB * kFewBlocks * 4;
+  static constexpr int FIT = (232448 - 1024 - 2 * SCALE_BYTES - 4 * NB * 4 - 512) / (B_BYTES + X_BYTES);
+  static constexpr int STAGES = FIT > 12 ? 12 : FIT;
+  static constexpr int PARTS = 4;                            // partial buffers
+  static constexpr int NCOLS = PARTS * NB;                   // 64 or 128
+  static constexpr int off_x = STAGES * B_BYTES;
+  static constexpr int off_scale = off_x + STAGES * X_BYTES;
+  static constexpr int off_max = off_scale + 2 * SCALE_BYTES;
+  static constexpr int off_bar = off_max + 4 * NB * 4;
+  static constexpr int total = off_bar + (2 * STAGES + 2 * PARTS) * 8 + 16;
+};
+
+struct FewArgs {
+  int n_items, k_blocks;       // work items of a row tile, K blocks
+  int experts_n;               // weight rows of an expert
+  int scale_rows;              // rows of an expert's weight scales
+  int up_tiles;                // GLU: 128-row tiles from a gate tile to its up tile
+  const float* x_scale;        // [M, k_blocks]
+  const float* w_scale;        // [experts, scale_rows, k_blocks]
+  void* c;                     // 16-bit [M, ldc], or GLU: e4m3 [M, ldc]
+  float* c_scale;              // GLU: [M, n_items]
+  int ldc, bf16;
+  const int32_t* tile_expert;  // [M / NB]
+  const int32_t* live;         // row tiles that have rows
+  int* status;
+};
+
+template <int NB, bool GLU>
+__global__ void __launch_bounds__(kThreads, 1)
+gemm_fp8_block_few_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_constant__ CUtensorMap tma_x, const FewArgs args) {
+  using C = FewCfg<NB>;
+  constexpr int STAGES_ = C::STAGES, PARTS = C::PARTS;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const uint32_t s_base = smem_u32(smem);
+  const uint32_t bar_base = s_base + C::off_bar;
+  auto full_bar = [&](int s) { return bar_base + 8u * s; };
+  auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES_ + s); };
+  auto pfull_bar = [&](int s) { return bar_base + 8u * (2 * STAGES_ + s); };
+  auto pempty_bar = [&](int s) { return bar_base + 8u * (2 * STAGES_ + PARTS + s); };
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + C::off_bar + (2 * STAGES_ + 2 * PARTS) * 8);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int KB = args.k_blocks;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES_; ++s) {
+      mbar_init(full_bar(s), 1);
+      mbar_init(empty_bar(s), 1);
+    }
+    for (int s = 0; s < PARTS; ++s) {
+      mbar_init(pfull_bar(s), 1);
+      mbar_init(pempty_bar(s), 4);
+    }
+    *abort_flag = 0;
+    fence_barrier_init();
+    prefetch_tensormap(&tma_w);
+    prefetch_tensormap(&tma_x);
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), C::NCOLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  pdl_enter();
+  // neighbouring CTAs have neighbouring row tiles of the same weight tiles: an expert of several tiles is read once
+  const int live = *args.live, items = live * args.n_items;
+  constexpr int HALVES = GLU ? 2 : 1;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ TMA producer
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int item = blockIdx.x; item < items && !*abort_flag; item += gridDim.x) {
+        const int m = item % live, n = item / live;
+        const int expert = args.tile_expert[m];
+        if (expert < 0) break;   // (none among the live tiles)
+        for (int half = 0; half < HALVES; ++half) {
+          const int row = expert * args.experts_n + (n + half * args.up_tiles) * BN;
+          for (int kb = 0; kb < KB; ++kb) {
+            if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, args.status, 125)) break;
+            mbar_expect_tx(full_bar(stage), B_BYTES + C::X_BYTES);
+            tma_load_2d(s_base + stage * B_BYTES, &tma_w, full_bar(stage), kb * BK, row);
+            tma_load_2d(s_base + C::off_x + stage * C::X_BYTES, &tma_x, full_bar(stage), kb * BK, m * NB);
+            if (++stage == STAGES_) { stage = 0; phase ^= 1u; }
+          }
+        }
+      }
+      if (*abort_flag) {  // give copies that are still in flight time to land before the CTA exits
+        const uint64_t t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    if (lane == 0) {
+      int stage = 0, pb = 0;
+      uint32_t phase = 0, pphase = 0;
+      bool ok = true;
+      for (int item = blockIdx.x; item < items && ok && !*abort_flag; item += gridDim.x) {
+        if (args.tile_expert[item % live] < 0) break;
+        for (int kb = 0; kb < HALVES * KB; ++kb) {
+          if (!mbar_wait(full_bar(stage), phase, abort_flag, args.status, 126)) { ok = false; break; }
+          if (!mbar_wait(pempty_bar(pb), pphase ^ 1u, abort_flag, args.status, 127)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t w_s = s_base + stage * B_BYTES, x_s = s_base + C::off_x + stage * C::X_BYTES, d = tmem_base + pb * NB;
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            mma_f8f6f4(d, smem_desc_sw128(w_s + k * 32), smem_desc_sw128(x_s + k * 32), idesc_dense(0, 0, BN, NB), k != 0 ? 1u : 0u);
+          tc_commit(empty_bar(stage));
+          tc_commit(pfull_bar(pb));
+          if (++stage == STAGES_) { stage = 0; phase ^= 1u; }
+          if (++pb == PARTS) { pb = 0; pphase ^= 1u; }
+        }
+      }
+    }
+  } else {
+    // ------------------------------------------------------------------ promotion + store (warps 2..5)
+    const int q = warp & 3, r = q * 32 + lane, tid = threadIdx.x - 64;   // tensor-memory lane = weight row of the tile
+    int pb = 0, buf = 0;
+    uint32_t pphase = 0;
+    bool ok = true;
+    // the row scales of a tile, [K block][NB], one work item ahead
+    auto ask_scales = [&](int item, int to) {
+      if (item < items) {
+        const float* src = args.x_scale + (size_t)(item % live) * NB * KB;
+        const uint32_t dst = s_base + C::off_scale + to * C::SCALE_BYTES;
+        for (int i = tid; i < NB * KB; i += 128) {
+          const int m = i / KB, kb = i - m * KB;
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + (kb * NB + m) * 4), "l"(src + i) : "memory");
+        }
+      }
+    };
+    ask_scales(blockIdx.x, 0);
+    // After a wait that gave up, the items are still walked through, so that the four warps meet at every barrier.
+    for (int item = blockIdx.x; item < items; item += gridDim.x, buf ^= 1) {
+      const int m = item % live, n = item / live;
+      const int expert = args.tile_expert[m];
+      if (expert < 0) break;
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      asm volatile("bar.sync 1, 128;" ::: "memory");   // the scales are there, and the other buffer has been read
+      ask_scales(item + gridDim.x, buf ^ 1);
+      const float4* xs = reinterpret_cast<const float4*>(smem + C::off_scale + buf * C::SCALE_BYTES);
+      float acc[HALVES][NB];
+#pragma unroll
+      for (int half = 0; half < HALVES; ++half) {
+#pragma unroll
+        for (int e = 0; e < NB; ++e) acc[half][e] = 0.f;
+        const float* ws_row = args.w_scale + ((size_t)expert * args.scale_rows + n + half * args.up_tiles) * KB;
+        float w_next = __ldg(ws_row);
+        for (int kb = 0; kb < KB && ok; ++kb) {
+          const float w = w_next;
+          if (kb + 1 < KB) w_next = __ldg(ws_row + kb + 1);
+          if (!mbar_wait(pfull_bar(pb), pphase, abort_flag, args.status, 128)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(pb * NB);
+          constexpr int W = NB == 16 ? 16 : 32;
+          uint32_t v[NB / W][W];
+#pragma unroll
+          for (int c = 0; c < NB / W; ++c) {
+            if constexpr (W == 16) tmem_ld_32x32b_x16(t_addr, v[c]);
+            else tmem_ld_32x32b_x32(t_addr + c * W, v[c]);
+          }
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < NB; e += 4) {
+            const float4 s = xs[kb * (NB / 4) + e / 4];
+            acc[half][e] = fmaf(__uint_as_float(v[e / W][e % W]), s.x * w, acc[half][e]);
+            acc[half][e + 1] = fmaf(__uint_as_float(v[e / W][e % W + 1]), s.y * w, acc[half][e + 1]);
+            acc[half][e + 2] = fmaf(__uint_as_float(v[e / W][e % W + 2]), s.z * w, acc[half][e + 2]);
+            acc[half][e + 3] = fmaf(__uint_as_float(v[e / W][e % W + 3]), s.w * w, acc[half][e + 3]);
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(pempty_bar(pb));
+          if (++pb == PARTS) { pb = 0; pphase ^= 1u; }
+        }
+      }
+      if (GLU) {
+        // rounded where the 16-bit form rounds; one maximum per column over the four warps
+        float* red = reinterpret_cast<float*>(smem + C::off_max);
+        auto round16 = [&](float x) {
+          return args.bf16 ? __bfloat162float(__float2bfloat16_rn(x)) : __half2float(__float2half_rn(x));
+        };
+#pragma unroll
+        for (int e = 0; e < NB; ++e) {
+          const float g = round16(acc[0][e]), u = round16(acc[HALVES - 1][e]), h = 0.5f * g;
+          float t;
+          asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(h));
+          acc[0][e] = round16(fmaf(h, t, h) * u);
+          const float mx = warp_max(fabsf(acc[0][e]));
+          if (lane == (e & 31)) red[q * NB + e] = mx;
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        uint8_t* const out = reinterpret_cast<uint8_t*>(args.c) + (size_t)m * NB * args.ldc + n * BN + r;
+#pragma unroll
+        for (int e = 0; e < NB; ++e) {
+          const float mx = fmaxf(fmaxf(red[e], red[NB + e]), fmaxf(red[2 * NB + e], red[3 * NB + e]));
+          const float scale = fmaxf(mx, 1e-8f) / kFp8Max;
+          if (ok) out[(size_t)e * args.ldc] = float_to_e4m3(acc[0][e] * (1.0f / scale));
+          if (ok && tid == e) args.c_scale[((size_t)m * NB + e) * args.n_items + n] = scale;
+        }
+        // (the next item writes `red` behind another barrier)
+      } else if (ok) {
+        // neighbouring lanes swap every other value, so that a lane stores two neighbouring columns of C at once
+        const int odd = lane & 1;
+        uint16_t* const p = reinterpret_cast<uint16_t*>(args.c) + (size_t)(m * NB + odd) * args.ldc + n * BN + (r & ~1);
+#pragma unroll
+        for (int e = 0; e < NB; e += 2) {
+          const float other = __shfl_xor_sync(0xffffffffu, odd ? acc[0][e] : acc[0][e + 1], 1);
+          const float lo = odd ? other : acc[0][e], hi = odd ? acc[0][e + 1] : other;
+          uint32_t w;
+          if (args.bf16) {
+            const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+            w = *reinterpret_cast<const uint32_t*>(&v);
+          } else {
+            const __half2 v = __floats2half2_rn(lo, hi);
+            w = *reinterpret_cast<const uint32_t*>(&v);
+          }
+          *reinterpret_cast<uint32_t*>(p + (size_t)e * args.ldc) = w;
+        }
+      }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, C::NCOLS);
+  }
+}
+
 struct MapKey {
   const void* ptr;
   uint64_t inner, rows;
@@ -392,8 +648,68 @@ MSGL_API int msgl_gemm_fp8_block(const void* a, long long lda, const void* b, vo
   return MSGL_OK;
 }
 
+namespace {
+template <int NB, bool GLU>
+int launch_few(const CUtensorMap& mw, const CUtensorMap& mx, const FewArgs& args, int ctas, cudaStream_t stream) {
+  constexpr int smem = FewCfg<NB>::total + 1024;
+  static_assert(smem <= 232448, "shared memory");
+  static const cudaError_t configured =
+      cudaFuncSetAttribute(gemm_fp8_block_few_kernel<NB, GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t e = configured;
+  if (e == cudaSuccess) e = msgl_launch(gemm_fp8_block_few_kernel<NB, GLU>, dim3(ctas), dim3(kThreads), smem, stream, mw, mx, args);
+  if (e != cudaSuccess) { msgl_set_error("gemm_fp8_block_few", e); return MSGL_CUDA_ERROR; }
+  return MSGL_OK;
+}
+}  // namespace
+
+// Grouped, few rows per expert: rows of a [M, K] e4m3 sorted by expert in tiles of nb = 16 or 32, live [1] the number of
+// tiles that have rows. glu 0: c 16-bit [M, N]. glu 1: N = 2 * inter rows of gate, then up; c e4m3 [M, inter] of
+// SiLU(gate) * up with c_scale [M, inter / 128]; dtype: the 16-bit type that gate, up and their product are rounded to.
+// N (inter) a multiple of 128, K of 128 up to 4096.
+MSGL_API int msgl_gemm_fp8_block_few(const void* a, const void* b, void* c, void* c_scale, int M, int N, int K, const void* a_scale,
+                                     const void* w_scale, const void* tile_expert, const void* live, int num_experts, int nb, int glu,
+                                     int dtype, cudaStream_t stream) {
+  if (M < 0 || N <= 0 || K <= 0 || K % 128 || K > 128 * kFewBlocks || N % (glu ? 256 : 128) || num_experts <= 0) return MSGL_BAD_ARG;
+  if ((nb != 16 && nb != 32) || M % nb || (glu && c_scale == nullptr)) return MSGL_BAD_ARG;
+  if (dtype != MSGL_BF16 && dtype != MSGL_F16) return MSGL_BAD_ARG;
+  if ((uintptr_t)a % 16 || (uintptr_t)b % 16 || (uintptr_t)c % 16) return MSGL_BAD_ARG;
+  if (M == 0) return MSGL_OK;
+  FewArgs args;
+  args.n_items = N / (glu ? 256 : 128);
+  args.k_blocks = K / 128;
+  args.experts_n = N;
+  args.scale_rows = N / 128;
+  args.up_tiles = args.n_items;
+  args.x_scale = (const float*)a_scale;
+  args.w_scale = (const float*)w_scale;
+  args.c = c;
+  args.c_scale = (float*)c_scale;
+  args.ldc = glu ? N / 2 : N;
+  args.bf16 = dtype == MSGL_BF16;
+  args.tile_expert = (const int32_t*)tile_expert;
+  args.live = (const int32_t*)live;
+  int* status = nullptr;
+  cudaGetSymbolAddress((void**)&status, g_block_status);
+  args.status = status;
+  CUtensorMap mw, mx;
+  int rc = make_map(&mw, b, (uint64_t)K, (uint64_t)N * num_experts, (uint64_t)K, BN, true);
+  if (rc == MSGL_OK) rc = make_map(&mx, a, (uint64_t)K, (uint64_t)M, (uint64_t)K, nb, false);
+  if (rc) return rc;
+  static int sms = 0;
+  if (sms == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (sms <= 0) sms = 148;
+  }
+  const long long most = (long long)(M / nb) * args.n_items;
+  const int ctas = most < sms ? (int)most : sms;
+  if (glu) return nb == 16 ? launch_few<16, true>(mw, mx, args, ctas, stream) : launch_few<32, true>(mw, mx, args, ctas, stream);
+  return nb == 16 ? launch_few<16, false>(mw, mx, args, ctas, stream) : launch_few<32, false>(mw, mx, args, ctas, stream);
+}
+
 // 0 when no bounded wait of the block-fp8 GEMM has run out since the last reset; else 121 producer /
-// 122 partial buffer / 123 stage / 124 promotion wait.
+// 122 partial buffer / 123 stage / 124 promotion wait (few rows: 125 / 127 / 126 / 128).
 MSGL_API int msgl_gemm_fp8_block_status(int reset) {
   int v = 0;
   cudaMemcpyFromSymbol(&v, g_block_status, sizeof(int));

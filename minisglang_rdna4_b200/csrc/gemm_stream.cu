@@ -306,6 +306,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
     asm volatile("bar.sync 1, 128;" ::: "memory");
     int acc = 0;
     uint32_t acc_phase = 0;
+    bool ok = true;
     for (int u = u_begin; u < u_end;) {
       const int tile = u / KB, kb0 = u - tile * KB, kb1 = min(KB, kb0 + u_end - u);
       const int n = tile * kTile + r;
@@ -319,7 +320,8 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
                  : args.bias_dtype == MSGL_F16 ? __half2float(reinterpret_cast<const __half*>(args.bias)[n])
                                                : reinterpret_cast<const float*>(args.bias)[n];
       }
-      if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag, args.status, 134)) break;
+      // after a wait that gave up, the range is still walked through, so that the four warps meet at every barrier
+      ok = ok && mbar_wait(tfull_bar(acc), acc_phase, abort_flag, args.status, 134);
       tc_fence_after();
       const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * NB);
       if (args.planes > 0) {

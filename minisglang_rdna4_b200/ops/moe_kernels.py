@@ -14,6 +14,7 @@ _lib.bind("msgl_moe_route", c_i, [c_p] * 5 + [c_i] * 5 + [c_f, c_i, c_i, c_ll, c
 _lib.bind("msgl_moe_combine32", c_i, [c_p, c_p, c_p, c_p, c_i, c_p, c_ll, c_p, c_i, c_i, c_i, c_i, c_p])
 _lib.bind("msgl_gemm_f32_grouped", c_i, [c_p, c_p, c_p, c_i, c_i, c_i, c_p, c_p])
 _lib.bind("msgl_moe_align", c_i, [c_p, c_p, c_p, c_p, c_p, c_p, c_p, c_p, c_i, c_i, c_i, c_i, c_i, c_i, c_p])
+_lib.bind("msgl_gemm_fp8_block_few", c_i, [c_p] * 4 + [c_i] * 3 + [c_p] * 4 + [c_i] * 4 + [c_p])
 _lib.bind("msgl_moe_quant_rows", c_i, [c_p] * 4 + [c_i] * 5 + [c_p])
 _lib.bind("msgl_moe_permute", c_i, [c_p, c_p, c_p, c_i, c_i, c_i, c_p, c_i, c_p])
 _lib.bind("msgl_moe_combine", c_i, [c_p, c_p, c_p, c_p, c_i, c_i, c_i, c_i, c_p])
@@ -44,38 +45,39 @@ def moe_route(router_logits, top_k, renormalize, scoring="softmax", scale=1.0, c
     return w, ids
 
 
-def max_sorted_rows(tokens: int, top_k: int, e_local: int) -> int:
-    rows = tokens * top_k + e_local * (BLOCK - 1)
-    return (rows + BLOCK - 1) // BLOCK * BLOCK
+def max_sorted_rows(tokens: int, top_k: int, e_local: int, block: int = BLOCK) -> int:
+    pairs = tokens * top_k
+    rows = pairs + min(e_local, pairs) * (block - 1)      # a tile that is not full for every expert that has rows
+    return (rows + block - 1) // block * block
 
 
-def moe_align(topk_ids, e_start: int, e_local: int, counts=None):
-    """Returns ``(sorted_pair [R], pair_row [T*k], tile_expert [R/128], meta [2])`` with R the
+def moe_align(topk_ids, e_start: int, e_local: int, counts=None, block: int = BLOCK):
+    """Returns ``(sorted_pair [R], pair_row [T*k], tile_expert [R/block], meta [2])`` with R the
     worst-case padded row count (static for a given T, k, E). ``counts`` = tokens per local expert
     when the routing kernel already produced them."""
     t, k = topk_ids.shape
     dev = topk_ids.device
-    rows = max_sorted_rows(t, k, e_local)
+    rows = max_sorted_rows(t, k, e_local, block)
     if counts is None and t * k > SMALL_PAIRS:
         counts = torch.zeros(e_local, dtype=torch.int32, device=dev)
         flat = topk_ids.reshape(-1).long() - e_start
         ok = (flat >= 0) & (flat < e_local)
         counts.index_add_(0, flat.clamp(0, e_local - 1), ok.to(torch.int32))
-    return _align_with_counts(topk_ids, counts, e_start, e_local, rows)
+    return _align_with_counts(topk_ids, counts, e_start, e_local, rows, block)
 
 
-def _align_with_counts(topk_ids, counts, e_start, e_local, rows):
+def _align_with_counts(topk_ids, counts, e_start, e_local, rows, block):
     t, k = topk_ids.shape
     dev = topk_ids.device
     offsets = torch.empty(e_local + 1, dtype=torch.int32, device=dev)
     cursor = torch.empty(e_local, dtype=torch.int32, device=dev)
-    tile_expert = torch.empty(rows // BLOCK, dtype=torch.int32, device=dev)
+    tile_expert = torch.empty(rows // block, dtype=torch.int32, device=dev)
     meta = torch.empty(2, dtype=torch.int32, device=dev)
     sorted_pair = torch.empty(rows, dtype=torch.int32, device=dev)
     pair_row = torch.empty(t * k, dtype=torch.int32, device=dev)
     check(lib().msgl_moe_align(topk_ids.data_ptr(), K._p(counts), offsets.data_ptr(), cursor.data_ptr(),
                                tile_expert.data_ptr(), meta.data_ptr(), sorted_pair.data_ptr(), pair_row.data_ptr(),
-                               t, k, e_start, e_local, rows, BLOCK, K._stream()), "moe_align")
+                               t, k, e_start, e_local, rows, block, K._stream()), "moe_align")
     if t * k <= SMALL_PAIRS:
         K._count("moe_align", "moe_align_small_kernel")
     else:
@@ -254,6 +256,38 @@ def quantise_sorted(kind: str, x, pair_row, rows: int, k: int):
     return q, s
 
 
+def few_rows_block(pairs: int, experts: int, two_inter: int, hidden: int) -> int:
+    """Rows of a tile for ``gemm_fp8_block_few``, 0 where the 128-row tiles of ``gemm_fp8_block`` are taken: enough for the rows
+    that an expert has on average with room to spare (a second tile reads the expert's weights again, from L2). B200, 128
+    experts of 2048 x 768, us a layer with tiles of 16 / 32 / 128 rows: 8 rows on average 151 / 179 / 211, 16 195 / 182 / 224, 20
+    235 / 184 / 222, 32 309 / 243 / 219."""
+    if two_inter % 256 or hidden % 128 or max(two_inter // 2, hidden) > 4096:
+        return 0
+    mean = pairs / experts
+    return 16 if mean <= 12 else 32 if mean <= 24 else 0
+
+
+def gemm_fp8_block_few(a_q, a_scale, b_q, b_scale, tile_expert, meta, block, dtype, glu=False):
+    """The grouped block-fp8 product for few rows per expert: ``a_q [R, K]`` e4m3 rows sorted by expert in tiles of ``block``
+    (``moe_align``) with ``a_scale [R, K/128]``, ``b_q [E, N, K]``, ``b_scale [E, N/128, K/128]`` -> ``[R, N]`` of ``dtype``;
+    ``glu``: ``(e4m3 [R, N/2], scales [R, N/256])`` of SiLU(gate) * up, gate and up rounded to ``dtype`` first."""
+    e, n, k = b_q.shape
+    r = a_q.shape[0]
+    assert a_q.is_contiguous() and b_q.is_contiguous() and a_scale.is_contiguous() and b_scale.is_contiguous()
+    assert a_scale.dtype == b_scale.dtype == torch.float32 and a_q.shape[1] == k and b_scale.shape == (e, n // 128, k // 128)
+    out_s = None
+    if glu:
+        out = torch.empty((r, n // 2), dtype=torch.float8_e4m3fn, device=a_q.device)
+        out_s = torch.empty((r, n // 256), dtype=torch.float32, device=a_q.device)
+    else:
+        out = torch.empty((r, n), dtype=dtype, device=a_q.device)
+    check(lib().msgl_gemm_fp8_block_few(a_q.data_ptr(), b_q.data_ptr(), out.data_ptr(), K._p(out_s), r, n, k, a_scale.data_ptr(),
+                                        b_scale.data_ptr(), tile_expert.data_ptr(), meta.data_ptr(), e, block, int(glu), _DT[dtype],
+                                        K._stream()), "gemm_fp8_block_few")
+    K._count("gemm_w8a8_block_grouped", "gemm_fp8_block_few_kernel")
+    return (out, out_s) if glu else out
+
+
 def run_experts_q(kind: str, xq, xsc, tile_expert, weights, out_dtype, sorted_pair=None):
     """The two expert GEMMs with SiLU·mul (+ re-quantisation) between them, on expert-sorted rows
     that are already in the input form of ``kind`` (``quantise_rows``): 16-bit rows for ``bf16``,
@@ -288,6 +322,14 @@ def moe_forward_quant(kind: str, x, weights, topk_w, topk_ids, expert_offset=0, 
     for quantised expert stacks ``weights`` of ``kind``."""
     e_local = weights[0].shape[0]
     k = topk_ids.shape[1]
+    block = few_rows_block(x.shape[0] * k, e_local, weights[0].shape[1], x.shape[1]) if kind == "fp8_block" else 0
+    if block:
+        q13, s13, q2, s2 = weights
+        sorted_pair, pair_row, tile_expert, meta = moe_align(topk_ids, expert_offset, e_local, counts, block)
+        xq, xsc = quantise_sorted(kind, x, pair_row, sorted_pair.numel(), k)
+        aq, asc = gemm_fp8_block_few(xq, xsc, q13, s13, tile_expert, meta, block, x.dtype, glu=True)
+        y = gemm_fp8_block_few(aq, asc, q2, s2, tile_expert, meta, block, x.dtype)
+        return _combine(y, topk_w, pair_row, x, k)
     sorted_pair, pair_row, tile_expert, _meta = moe_align(topk_ids, expert_offset, e_local, counts)
     if ROW_QUANT[kind] == 0:
         y = run_experts(kind, _permute(x, sorted_pair, k), tile_expert, weights, x.dtype)
