@@ -12,13 +12,20 @@
 // The scales change every 128 elements of K and are arbitrary fp32 numbers, so they cannot ride
 // on the block-scaled MMA kinds (those take power-of-two UE8M0 scales). Instead every K block
 // (= one pipeline stage, four tcgen05.mma kind::f8f6f4 of K = 32) is accumulated on its own
-// into one of two 128-column tensor-memory buffers; the four promotion warps pull a finished
-// block out with tcgen05.ld, multiply by the block's scale product and add it to a 128-float
-// register accumulator per row while the tensor core already works on the next block in the
-// other buffer. Every row's sum runs over K in ascending order and does not depend on M.
+// into one of four 128-column tensor-memory buffers; the eight promotion warps pull a finished
+// block out with tcgen05.ld, multiply by the block's scale product and add it to a 64-float
+// register accumulator per row and half while the tensor core already works on the next blocks in the
+// other buffers. Every row's sum runs over K in ascending order and does not depend on M.
 //
 // Structure as in gemm_tcgen05.cu: persistent CTAs, warp 0 = TMA producer, warp 1 = MMA issuer
-// and tensor-memory owner, warps 2-5 = promotion + store. All waits are bounded.
+// and tensor-memory owner, warps 2-9 = promotion + store. All waits are bounded.
+//
+// Bound of many rows: what an SM takes in from L2, 32 KB for each K block of a tile (with the MMAs, the promotion and the stores all
+// left out a block still takes 0.49 us, 65 GB/s an SM). On top of that came the stores: a lane wrote 16 bytes of its own row at a time,
+// a quarter of the time of the first product and 30 % of the second. A warp now packs its 32 x 64 results into shared memory and
+// leaves them to one TMA store, whose end it waits for before the next tile's. B200, 4480 tokens with 8 of 128 experts, us:
+// N 1536, K 2048 326 -> 270, N 2048, K 768 181 -> 135; 1024 tokens, the whole layer 236 -> 211. (Eight promotion warps in the place of four and
+// four partial buffers in the place of two changed nothing by themselves; they make room for the stores.)
 #include "common.cuh"
 #include "ptx.cuh"
 
@@ -34,15 +41,19 @@ int msgl_b_static_level();   // gemm_tcgen05.cu: level set by msgl_gemm_static_w
 namespace {
 
 constexpr int BM = 128, BN = 128, BK = 128;
-constexpr int kThreads = 192;
-constexpr int STAGES = 6;
+constexpr int kThreads = 320;      // TMA, MMA, eight promotion warps
+constexpr int kFewThreads = 192;   // four promotion warps
+constexpr int PARTS = 4;           // partial buffers
+constexpr int STAGES = 5;
 constexpr int A_BYTES = BM * BK, B_BYTES = BN * BK;
 constexpr int off_a = 0;
 constexpr int off_b = off_a + STAGES * A_BYTES;
-constexpr int off_bar = off_b + STAGES * B_BYTES;
-constexpr int n_bars = 2 * STAGES + 4;  // full / empty per stage, pfull / pempty per partial buffer
+constexpr int PATCH_BYTES = 32 * 128;   // a promotion warp's results: 32 rows of 64 16-bit columns
+constexpr int off_patch = off_b + STAGES * B_BYTES;
+constexpr int off_bar = off_patch + 8 * PATCH_BYTES;
+constexpr int n_bars = 2 * STAGES + 2 * PARTS;  // full / empty per stage, pfull / pempty per partial buffer
 constexpr int smem_total = off_bar + n_bars * 8 + 16;
-constexpr int NCOLS = 256;
+constexpr int NCOLS = PARTS * BN;
 
 struct BlockArgs {
   int M, N, K;
@@ -53,6 +64,7 @@ struct BlockArgs {
   long long ldc;
   int out_dtype;
   const int32_t* tile_expert;  // grouped: expert of M tile m (negative: tile past the live rows)
+  int tma_out;                 // results leave through tma_c
   int l2_ahead;                // request a work item's weight stream into L2 one item ahead
   int* status;
 };
@@ -61,7 +73,7 @@ __device__ int g_block_status = 0;
 
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
-                      const BlockArgs args) {
+                      const __grid_constant__ CUtensorMap tma_c, const BlockArgs args) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t s_base = smem_u32(smem);
@@ -69,7 +81,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
   auto pfull_bar = [&](int s) { return bar_base + 8u * (2 * STAGES + s); };
-  auto pempty_bar = [&](int s) { return bar_base + 8u * (2 * STAGES + 2 + s); };
+  auto pempty_bar = [&](int s) { return bar_base + 8u * (2 * STAGES + PARTS + s); };
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + off_bar + n_bars * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + off_bar + n_bars * 8 + 4);
 
@@ -81,9 +93,9 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), 1);
     }
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < PARTS; ++s) {
       mbar_init(pfull_bar(s), 1);
-      mbar_init(pempty_bar(s), 4);
+      mbar_init(pempty_bar(s), 8);
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -160,13 +172,16 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
           tc_commit(empty_bar(stage));  // the stage is free once these MMAs have read it
           tc_commit(pfull_bar(pb));     // and this K block's partial sums are complete
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
-          if (++pb == 2) { pb = 0; pphase ^= 1u; }
+          if (++pb == PARTS) { pb = 0; pphase ^= 1u; }
         }
       }
     }
   } else {
-    // ------------------------------------------------------------------ promotion + store (warps 2..5)
-    const int q = warp & 3;  // tensor-memory lane quarter this warp may read
+    // ------------------------------------------------------------------ promotion + store (warps 2..9)
+    constexpr int W = BN / 2;
+    const int q = warp & 3;                  // tensor-memory lane quarter this warp may read
+    const int half = (warp - 2) >> 2;        // which 64 of the tile's 128 columns
+    const bool pairs = args.k_blocks % 2 == 0;   // row scales can be read two at a time
     int pb = 0;
     uint32_t pphase = 0;
     bool ok = true;
@@ -181,62 +196,87 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       const bool row_ok = row < args.M;
       const float* as_row = args.a_scale + (size_t)(row_ok ? row : 0) * args.k_blocks;
       const float* ws_row = args.w_scale + ((size_t)expert * args.n_tiles + n_tile) * args.k_blocks;
-      float acc[BN];
+      float as_odd = 0.f;
+      auto scale_of = [&](int kb) {   // asked for in ascending order
+        float a;
+        if (!pairs) {
+          a = __ldg(as_row + kb);
+        } else if ((kb & 1) == 0) {
+          const float2 two = __ldg(reinterpret_cast<const float2*>(as_row + kb));
+          a = two.x;
+          as_odd = two.y;
+        } else {
+          a = as_odd;
+        }
+        return row_ok ? a * __ldg(ws_row + kb) : 0.f;
+      };
+      float acc[W];
 #pragma unroll
-      for (int e = 0; e < BN; ++e) acc[e] = 0.f;
-      float s_next = row_ok ? __ldg(as_row) * __ldg(ws_row) : 0.f;
+      for (int e = 0; e < W; ++e) acc[e] = 0.f;
+      float s_next = scale_of(0);
       for (int kb = 0; kb < args.k_blocks; ++kb) {
         const float s = s_next;
-        if (kb + 1 < args.k_blocks) s_next = row_ok ? __ldg(as_row + kb + 1) * __ldg(ws_row + kb + 1) : 0.f;
+        if (kb + 1 < args.k_blocks) s_next = scale_of(kb + 1);
         if (!mbar_wait(pfull_bar(pb), pphase, abort_flag, args.status, 124)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(pb * BN);
-#pragma unroll
-        for (int c = 0; c < BN / 32; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(t_addr + c * 32, r);
-          tmem_ld_wait();
-#pragma unroll
-          for (int e = 0; e < 32; ++e) acc[c * 32 + e] = fmaf(__uint_as_float(r[e]), s, acc[c * 32 + e]);
-        }
+        const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(pb * BN + half * W);
+        uint32_t r0[32], r1[32];
+        tmem_ld_32x32b_x32(t_addr, r0);
+        tmem_ld_32x32b_x32(t_addr + 32, r1);
+        tmem_ld_wait();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(pempty_bar(pb));
-        if (++pb == 2) { pb = 0; pphase ^= 1u; }
+#pragma unroll
+        for (int e = 0; e < 32; ++e) {
+          acc[e] = fmaf(__uint_as_float(r0[e]), s, acc[e]);
+          acc[32 + e] = fmaf(__uint_as_float(r1[e]), s, acc[32 + e]);
+        }
+        if (++pb == PARTS) { pb = 0; pphase ^= 1u; }
       }
       if (!ok) break;
-      if (row_ok) {
-        const int colbase = n_tile * BN;
+      const int colbase = n_tile * BN + half * W;
+      auto pack = [&](int i) {   // columns 2i and 2i + 1
+        if (args.out_dtype == MSGL_BF16) {
+          __nv_bfloat162 v = __floats2bfloat162_rn(acc[2 * i], acc[2 * i + 1]);
+          return *reinterpret_cast<uint32_t*>(&v);
+        }
+        __half2 v = __floats2half2_rn(acc[2 * i], acc[2 * i + 1]);
+        return *reinterpret_cast<uint32_t*>(&v);
+      };
+      if (args.tma_out) {
+        uint8_t* const patch = smem + off_patch + (warp - 2) * PATCH_BYTES;
+        if (lane == 0) bulk_wait_group_read<0>();   // the tile before this one has left the patch
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < 8; ++u)   // 128-byte swizzle: 16-byte unit u of row r lives at unit u ^ (r & 7)
+          *reinterpret_cast<uint4*>(patch + lane * 128 + ((u ^ (lane & 7)) << 4)) =
+              make_uint4(pack(u * 4), pack(u * 4 + 1), pack(u * 4 + 2), pack(u * 4 + 3));
+        fence_proxy_async();
+        __syncwarp();
+        const int row0 = m_tile * BM + q * 32;
+        if (lane == 0 && row0 < args.M && colbase < args.N) {
+          tma_store_2d(&tma_c, s_base + off_patch + (warp - 2) * PATCH_BYTES, colbase, row0);
+          bulk_commit_group();
+        }
+      } else if (row_ok) {
         if (args.out_dtype == MSGL_F32) {
           float* crow = reinterpret_cast<float*>(args.c) + (size_t)row * args.ldc + colbase;
 #pragma unroll
-          for (int g = 0; g < BN / 4; ++g)
+          for (int g = 0; g < W / 4; ++g)
             if (colbase + g * 4 < args.N)
               *reinterpret_cast<float4*>(crow + g * 4) =
                   make_float4(acc[g * 4], acc[g * 4 + 1], acc[g * 4 + 2], acc[g * 4 + 3]);
         } else {
           uint16_t* crow = reinterpret_cast<uint16_t*>(args.c) + (size_t)row * args.ldc + colbase;
-          const bool bf = args.out_dtype == MSGL_BF16;
 #pragma unroll
-          for (int g = 0; g < BN / 8; ++g) {
-            if (colbase + g * 8 < args.N) {
-              uint32_t w[4];
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                if (bf) {
-                  __nv_bfloat162 v = __floats2bfloat162_rn(acc[g * 8 + 2 * e], acc[g * 8 + 2 * e + 1]);
-                  w[e] = *reinterpret_cast<uint32_t*>(&v);
-                } else {
-                  __half2 v = __floats2half2_rn(acc[g * 8 + 2 * e], acc[g * 8 + 2 * e + 1]);
-                  w[e] = *reinterpret_cast<uint32_t*>(&v);
-                }
-              }
-              *reinterpret_cast<uint4*>(crow + g * 8) = make_uint4(w[0], w[1], w[2], w[3]);
-            }
-          }
+          for (int g = 0; g < W / 8; ++g)
+            if (colbase + g * 8 < args.N)
+              *reinterpret_cast<uint4*>(crow + g * 8) = make_uint4(pack(g * 4), pack(g * 4 + 1), pack(g * 4 + 2), pack(g * 4 + 3));
         }
       }
     }
+    if (lane == 0) bulk_wait_group<0>();
   }
 
   tc_fence_before();
@@ -299,8 +339,9 @@ __global__ void __launch_bounds__(256) silu_mul_quant_group_kernel(const T* __re
 // the 128 up rows that belong to them, so SiLU(gate) * up, and its maximum over the group of 128 outputs, are at hand in the
 // registers of one warpgroup, and e4m3 rows leave the kernel in the place of 16-bit ones that a kernel of its own read again.
 // B200, us of a whole expert layer (8 of 128 experts, 2048 columns, 768 wide; the weights alone take 92), 128-row tiles -> this:
-// 1 token 31.7 -> 34.3, 4: 66.6 -> 61.4, 16: 157 -> 109, 48: 203 -> 135, 128: 211 -> 151, 256 (NB 32): 224 -> 182, 320: 222 -> 184. Tiles of
-// 64 rows took 280.
+// 1 token 30.7 -> 31.2, 4: 60.4 -> 56.8, 16: 135 -> 98, 48: 172 -> 124, 128: 179 -> 137, 256 (NB 32): 188 -> 152, 320: 183 -> 154. The epilogue
+// of GLU is a chain that the ring covers up to NB = 32 only (the divisions by one thread a column and the maxima in one
+// instruction took 30 us off at NB = 32): tiles of 64 rows took 280.
 // ------------------------------------------------------------------------------------------
 constexpr int kFewBlocks = 32;     // K blocks, at most
 
@@ -309,7 +350,6 @@ template <int NB> struct FewCfg {
   static constexpr int SCALE_BYTES = NB * kFewBlocks * 4;
   static constexpr int FIT = (232448 - 1024 - 2 * SCALE_BYTES - 4 * NB * 4 - 512) / (B_BYTES + X_BYTES);
   static constexpr int STAGES = FIT > 12 ? 12 : FIT;
-  static constexpr int PARTS = 4;                            // partial buffers
   static constexpr int NCOLS = PARTS * NB;                   // 64 or 128
   static constexpr int off_x = STAGES * B_BYTES;
   static constexpr int off_scale = off_x + STAGES * X_BYTES;
@@ -334,10 +374,10 @@ struct FewArgs {
 };
 
 template <int NB, bool GLU>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kFewThreads, 1)
 gemm_fp8_block_few_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_constant__ CUtensorMap tma_x, const FewArgs args) {
   using C = FewCfg<NB>;
-  constexpr int STAGES_ = C::STAGES, PARTS = C::PARTS;
+  constexpr int STAGES_ = C::STAGES;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t s_base = smem_u32(smem);
@@ -463,28 +503,24 @@ gemm_fp8_block_few_kernel(const __grid_constant__ CUtensorMap tma_w, const __gri
         for (int kb = 0; kb < KB && ok; ++kb) {
           const float w = w_next;
           if (kb + 1 < KB) w_next = __ldg(ws_row + kb + 1);
+          float sw[NB];   // ready before the block is
+#pragma unroll
+          for (int e = 0; e < NB; e += 4) {
+            const float4 x = xs[kb * (NB / 4) + e / 4];
+            sw[e] = x.x * w; sw[e + 1] = x.y * w; sw[e + 2] = x.z * w; sw[e + 3] = x.w * w;
+          }
           if (!mbar_wait(pfull_bar(pb), pphase, abort_flag, args.status, 128)) { ok = false; break; }
           tc_fence_after();
           const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(pb * NB);
-          constexpr int W = NB == 16 ? 16 : 32;
-          uint32_t v[NB / W][W];
-#pragma unroll
-          for (int c = 0; c < NB / W; ++c) {
-            if constexpr (W == 16) tmem_ld_32x32b_x16(t_addr, v[c]);
-            else tmem_ld_32x32b_x32(t_addr + c * W, v[c]);
-          }
+          uint32_t v[NB];
+          if constexpr (NB == 16) tmem_ld_32x32b_x16(t_addr, v);
+          else tmem_ld_32x32b_x32(t_addr, v);
           tmem_ld_wait();
-#pragma unroll
-          for (int e = 0; e < NB; e += 4) {
-            const float4 s = xs[kb * (NB / 4) + e / 4];
-            acc[half][e] = fmaf(__uint_as_float(v[e / W][e % W]), s.x * w, acc[half][e]);
-            acc[half][e + 1] = fmaf(__uint_as_float(v[e / W][e % W + 1]), s.y * w, acc[half][e + 1]);
-            acc[half][e + 2] = fmaf(__uint_as_float(v[e / W][e % W + 2]), s.z * w, acc[half][e + 2]);
-            acc[half][e + 3] = fmaf(__uint_as_float(v[e / W][e % W + 3]), s.w * w, acc[half][e + 3]);
-          }
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(pempty_bar(pb));
+#pragma unroll
+          for (int e = 0; e < NB; ++e) acc[half][e] = fmaf(__uint_as_float(v[e]), sw[e], acc[half][e]);
           if (++pb == PARTS) { pb = 0; pphase ^= 1u; }
         }
       }
@@ -500,17 +536,23 @@ gemm_fp8_block_few_kernel(const __grid_constant__ CUtensorMap tma_w, const __gri
           float t;
           asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(h));
           acc[0][e] = round16(fmaf(h, t, h) * u);
-          const float mx = warp_max(fabsf(acc[0][e]));
-          if (lane == (e & 31)) red[q * NB + e] = mx;
+          // (bits of magnitudes sort as the magnitudes do; fmaxf would leave a NaN out too)
+          const float a = fabsf(acc[0][e]);
+          const uint32_t mx = __reduce_max_sync(0xffffffffu, a == a ? __float_as_uint(a) : 0u);
+          if (lane == (e & 31)) red[q * NB + e] = __uint_as_float(mx);
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (tid < NB) {   // one thread per column divides
+          const float mx = fmaxf(fmaxf(red[tid], red[NB + tid]), fmaxf(red[2 * NB + tid], red[3 * NB + tid]));
+          const float scale = fmaxf(mx, 1e-8f) / kFp8Max;
+          if (ok) args.c_scale[((size_t)m * NB + tid) * args.n_items + n] = scale;
+          red[tid] = 1.0f / scale;
         }
         asm volatile("bar.sync 1, 128;" ::: "memory");
         uint8_t* const out = reinterpret_cast<uint8_t*>(args.c) + (size_t)m * NB * args.ldc + n * BN + r;
+        if (ok) {
 #pragma unroll
-        for (int e = 0; e < NB; ++e) {
-          const float mx = fmaxf(fmaxf(red[e], red[NB + e]), fmaxf(red[2 * NB + e], red[3 * NB + e]));
-          const float scale = fmaxf(mx, 1e-8f) / kFp8Max;
-          if (ok) out[(size_t)e * args.ldc] = float_to_e4m3(acc[0][e] * (1.0f / scale));
-          if (ok && tid == e) args.c_scale[((size_t)m * NB + e) * args.n_items + n] = scale;
+          for (int e = 0; e < NB; ++e) out[(size_t)e * args.ldc] = float_to_e4m3(acc[0][e] * red[e]);
         }
         // (the next item writes `red` behind another barrier)
       } else if (ok) {
@@ -627,7 +669,19 @@ MSGL_API int msgl_gemm_fp8_block(const void* a, long long lda, const void* b, vo
   if (rc) return rc;
   rc = make_map(&mb, b, (uint64_t)K, b_rows, (uint64_t)K, BN, true);
   if (rc) return rc;
+  // 16-bit results whose rows a tensor map can describe leave as 32 x 64 boxes
+  CUtensorMap mc = ma;
+  args.tma_out = out_dtype != MSGL_F32 && ldc % 8 == 0 && ldc >= N && (uintptr_t)c % 16 == 0;
+  if (args.tma_out) {
+    msgl_encode_tiled_fn enc = msgl_get_encode_tiled();
+    cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)M}, strides[1] = {(cuuint64_t)ldc * 2};
+    cuuint32_t box[2] = {64, 32}, estr[2] = {1, 1};
+    args.tma_out = enc != nullptr &&
+                   enc(&mc, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, c, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                       CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  }
   constexpr int smem = smem_total + 1024;
+  static_assert(smem <= 232448, "shared memory");
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(gemm_fp8_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -643,7 +697,7 @@ MSGL_API int msgl_gemm_fp8_block(const void* a, long long lda, const void* b, vo
   }
   int grid = args.m_tiles * args.n_tiles;
   if (grid > sms) grid = sms;
-  cudaError_t e = msgl_launch(gemm_fp8_block_kernel, dim3(grid), dim3(kThreads), smem, stream, ma, mb, args);
+  cudaError_t e = msgl_launch(gemm_fp8_block_kernel, dim3(grid), dim3(kThreads), smem, stream, ma, mb, mc, args);
   if (e != cudaSuccess) { msgl_set_error("gemm_fp8_block launch", e); return MSGL_CUDA_ERROR; }
   return MSGL_OK;
 }
@@ -656,7 +710,7 @@ int launch_few(const CUtensorMap& mw, const CUtensorMap& mx, const FewArgs& args
   static const cudaError_t configured =
       cudaFuncSetAttribute(gemm_fp8_block_few_kernel<NB, GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   cudaError_t e = configured;
-  if (e == cudaSuccess) e = msgl_launch(gemm_fp8_block_few_kernel<NB, GLU>, dim3(ctas), dim3(kThreads), smem, stream, mw, mx, args);
+  if (e == cudaSuccess) e = msgl_launch(gemm_fp8_block_few_kernel<NB, GLU>, dim3(ctas), dim3(kFewThreads), smem, stream, mw, mx, args);
   if (e != cudaSuccess) { msgl_set_error("gemm_fp8_block_few", e); return MSGL_CUDA_ERROR; }
   return MSGL_OK;
 }
