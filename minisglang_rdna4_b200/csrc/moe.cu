@@ -26,8 +26,9 @@ constexpr int kMaxExperts = 512;
 constexpr int kMaxTopK = 16;
 constexpr int kSmallPairs = 4096;   // (token, expert) pairs that one CTA aligns: eight a thread
 
-// one warp per token; E <= 512 (16 values per lane)
-template <typename T>
+// one warp per token; PER values per lane: E <= 32 PER. Each of the k rounds walks all PER values.
+// B200, us, 8 of 128 experts: 48 tokens 5.7 -> 3.5, 4480 tokens 16.0 -> 9.4; of 256: 5.8 -> 4.2, 16.1 -> 11.9; of 512 as before.
+template <typename T, int PER>
 __global__ void moe_route_kernel(const T* __restrict__ logits, const float* __restrict__ bias,
                                  float* __restrict__ topk_w, int32_t* __restrict__ topk_ids,
                                  int32_t* __restrict__ counts, int tokens, int E, int k, int renorm, int sigmoid,
@@ -36,7 +37,6 @@ __global__ void moe_route_kernel(const T* __restrict__ logits, const float* __re
   const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (t >= tokens) return;
   const int lane = threadIdx.x & 31;
-  constexpr int PER = kMaxExperts / 32;
   float v[PER];
   float mx = -INFINITY;
 #pragma unroll
@@ -431,8 +431,14 @@ MSGL_API int msgl_moe_route(const void* logits, const void* bias, void* topk_w, 
   if (tokens == 0) return MSGL_OK;
   const int warps = 4;
   const int blocks = (tokens + warps - 1) / warps;
-#define ROUTE(T)                                                                                                   \
-  msgl_launch(moe_route_kernel<T>, dim3(blocks), dim3(warps * 32), 0, stream, (const T*)logits, (const float*)bias, \
+#define ROUTE(T)                                  \
+  do {                                            \
+    if (E <= 128) ROUTE_PER(T, 4);                \
+    else if (E <= 256) ROUTE_PER(T, 8);           \
+    else ROUTE_PER(T, 16);                        \
+  } while (0)
+#define ROUTE_PER(T, PER)                                                                                            \
+  msgl_launch(moe_route_kernel<T, PER>, dim3(blocks), dim3(warps * 32), 0, stream, (const T*)logits, (const float*)bias, \
               (float*)topk_w, (int32_t*)topk_ids, (int32_t*)counts, tokens, E, k, renorm, sigmoid, scale, e_start,   \
               e_local, ld, groups, keep)
   if (dtype == MSGL_F32) ROUTE(float);
@@ -440,6 +446,7 @@ MSGL_API int msgl_moe_route(const void* logits, const void* bias, void* topk_w, 
   else if (dtype == MSGL_F16) ROUTE(__half);
   else return MSGL_BAD_ARG;
 #undef ROUTE
+#undef ROUTE_PER
   MSGL_CHECK_LAUNCH("moe_route");
   return MSGL_OK;
 }
