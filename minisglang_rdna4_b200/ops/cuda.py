@@ -259,12 +259,13 @@ def store_kv(k, v, k_cache, v_cache, out_loc, k_scale=None, v_scale=None):
 
 
 # ------------------------------------------------------------------------------------------ attention
-_KV_MAPS: Dict[Tuple, Tuple[np.ndarray, object]] = {}
+_KV_MAPS: Dict[Tuple, np.ndarray] = {}
 
 
 def _kv_map(k_cache: torch.Tensor):
     """TMA descriptor over the pool buffer that ``k_cache`` (one layer's K plane) is a view of.
-    Returns ``(descriptor bytes, layer index, number of layers)``."""
+    Returns ``(descriptor bytes, layer index, number of layers)``. A descriptor says no more than its key (address, shape, type), so
+    the pool itself is not kept: an engine that has been shut down gives its memory back."""
     base = k_cache._base if k_cache._base is not None else k_cache
     pages_p1, hk, ps, d = k_cache.shape
     if base.dim() == 6:
@@ -276,16 +277,15 @@ def _kv_map(k_cache: torch.Tensor):
     else:  # a stand-alone [pages, hk, ps, d] K tensor followed by nothing: treat as one layer
         raise ValueError("paged_attention expects k_cache / v_cache to be planes of one pool buffer")
     key = (root.data_ptr(), tuple(root.shape), root.dtype)
-    hit = _KV_MAPS.get(key)
-    if hit is None:
+    buf = _KV_MAPS.get(key)
+    if buf is None:
         buf = np.zeros(128, dtype=np.uint8)
         check(lib().msgl_attn_make_kv_map(buf.ctypes.data, root.data_ptr(), root.element_size(), d, ps, hk,
                                           pages_p1, 2 * layers), "attn_make_kv_map")
         if len(_KV_MAPS) > 512:            # layers with planes of their own have a map each
             _KV_MAPS.clear()
-        hit = (buf, root)
-        _KV_MAPS[key] = hit
-    return hit[0], layer, layers
+        _KV_MAPS[key] = buf
+    return buf, layer, layers
 
 
 def make_pool_buffer(num_layers, pages_plus_one, hk, page_size, d, dtype, device):

@@ -149,6 +149,21 @@ def test_graph_and_two_streams():
         assert torch.equal(y, want)
 
 
+def test_a_pool_is_given_back():
+    import gc
+
+    before = torch.cuda.memory_allocated()
+    c = _case([5000], 32, 8, 128, True)
+    one = torch.ones(8, device="cuda")
+    for deal in (True, False):
+        _run(c, True, scales=(one, one), deal=deal)
+    size = c[1].numel()
+    del c
+    gc.collect()
+    torch.cuda.synchronize()
+    assert torch.cuda.memory_allocated() - before < size
+
+
 def test_what_it_does_not_cover():
     from minisglang_rdna4_b200.ops._lib import lib
 
