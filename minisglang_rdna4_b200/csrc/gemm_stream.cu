@@ -528,6 +528,17 @@ MSGL_API int msgl_gemm_stream(int kind, const void* a, long long lda, const void
   }
 }
 
+// Number of the capture that a stream is in, 0 where it is in none: no two captures of a process have the same.
+MSGL_API unsigned long long msgl_capture_id(cudaStream_t stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(stream, &status, &id) != cudaSuccess) {   // the legacy stream while another one captures
+    cudaGetLastError();
+    return 0;
+  }
+  return status == cudaStreamCaptureStatusActive ? id : 0;
+}
+
 // 0 when no bounded wait has run out since the last reset; else 131 producer / 132 accumulator / 133 stage / 134 epilogue.
 MSGL_API int msgl_gemm_stream_status(int reset) {
   int v = 0;

@@ -56,6 +56,7 @@ _SIGNATURES = {
     "msgl_gemm_stream": (c_i, [c_i, c_p, c_ll, c_p, c_p, c_ll, c_i, c_i, c_i, c_p, c_p, c_p, c_i, c_p, c_i, c_i, c_i, c_p, c_p,
                                c_p]),
     "msgl_gemm_stream_status": (c_i, [c_i]),
+    "msgl_capture_id": (ctypes.c_ulonglong, [c_p]),
     "msgl_rms_norm_planes": (c_i, [c_p, c_i, c_p, c_p, c_p, c_p, c_p, c_i, c_i, c_f, c_i, c_i, c_p]),
     "msgl_gemm_status": (c_i, [c_i]),
     "msgl_gemm_pair_mode": (c_i, [c_i]),

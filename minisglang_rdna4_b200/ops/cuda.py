@@ -9,6 +9,7 @@ python/minisgl/_hip_engage.py:49-71).
 from __future__ import annotations
 
 import ctypes
+import threading
 from typing import Dict, Optional, Tuple
 
 import numpy as np
@@ -730,7 +731,10 @@ def take_pending_gemm_tp():
 
 
 _STREAM_PLANS: Dict[Tuple[int, int, int, bool], Tuple[int, int]] = {}
-_STREAM_COUNTERS: Dict[Tuple, list] = {}
+_STREAM_COUNTERS: Dict[Tuple, torch.Tensor] = {}            # by device and stream, the latest used last
+_CAPTURE_COUNTERS: Dict[Tuple, Tuple[int, list]] = {}       # by device and stream: (capture, its sets)
+_STREAM_COUNTERS_LOCK = threading.Lock()
+STREAM_COUNTER_SETS = 64
 STREAM_PLANES = 8
 
 
@@ -745,15 +749,37 @@ def _stream_plan(kind: int, n: int, k: int, planes: bool) -> Tuple[int, int]:
     return got
 
 
+def _capture_id(stream: int) -> int:
+    return int(lib().msgl_capture_id(stream))
+
+
 def _stream_counters(device, tiles: int) -> torch.Tensor:
-    """Arrival counters of the tiles that CTAs share: zero between calls. One set for each stream, and one for what is
-    captured on it, since calls on two streams may run side by side. A captured graph holds their address, so they stay
-    (16 KB each; streams come from a pool of fixed size)."""
-    key = (device, _stream(), torch.cuda.is_current_stream_capturing())
-    sets = _STREAM_COUNTERS.setdefault(key, [])
-    if not sets or sets[-1].numel() < tiles:
-        sets.append(workspace(f"GEMM tile counters {key[1:]} {len(sets)}", max(2 * tiles, 4096), torch.int32, device, zero=True))
-    return sets[-1]
+    """Arrival counters of the tiles that CTAs share: zero between calls. One set for each stream, since calls on two streams
+    may run side by side; the one of the stream that has gone longest without a call is dropped when there are many (its memory is the
+    allocator's for that stream, so what still runs there is done with it first).
+
+    A capture has sets of its own, zeroed by the graph in front of the first product that uses them: memory of a graph's
+    pool belongs to the other graphs of the pool too, graphs are replayed in any order and on any stream, and a fill that
+    is captured is not run. They are kept until the stream is in another capture: until then they must not be reused, after that they may."""
+    stream = _stream()
+    key, capture, numel = (device, stream), _capture_id(stream), max(2 * tiles, 4096)
+    with _STREAM_COUNTERS_LOCK:
+        if capture:
+            held = _CAPTURE_COUNTERS.get(key)
+            if held is None or held[0] != capture:
+                held = _CAPTURE_COUNTERS[key] = (capture, [])
+            if not held[1] or held[1][-1].numel() < tiles:
+                held[1].append(torch.zeros(numel, dtype=torch.int32, device=device))
+            return held[1][-1]
+        got = _STREAM_COUNTERS.pop(key, None)
+        if got is None or got.numel() < tiles:
+            got = workspace(f"GEMM tile counters {stream:#x}", numel, torch.int32, device, zero=True)
+        _STREAM_COUNTERS[key] = got
+        while len(_STREAM_COUNTERS) > STREAM_COUNTER_SETS:
+            old = next(iter(_STREAM_COUNTERS))
+            del _STREAM_COUNTERS[old]
+            _GUARDED.pop(f"GEMM tile counters {old[1]:#x}@{old[0]}", None)
+        return got
 
 
 def _stream_pays(m: int, weight_bytes: int, planes: bool) -> bool:

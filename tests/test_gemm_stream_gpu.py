@@ -83,6 +83,96 @@ def test_calls_on_two_streams_have_counters_of_their_own():
     assert all(torch.equal(o, outs[0]) for o in outs)
 
 
+def _shared_tiles(n, k):
+    """A product whose tiles several CTAs share, and its result."""
+    from minisglang_rdna4_b200.ops import cuda as K
+
+    (x, w, *_), _ = _operands("bf16", 8, n, k)
+    run = lambda: K._gemm_stream(1, x, w, 8, n, k, torch.float32, None, None, None, None, False)  # noqa: E731
+    return run, run()
+
+
+def _captured(run, stream, pool=None):
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, pool=pool, stream=stream):
+        y = run()
+    return graph, y
+
+
+@pytest.mark.parametrize("warm", [True, False])
+def test_graphs_of_one_pool_in_any_order(warm):
+    """A graph finds its counters at zero whatever ran before it: the pool's memory belongs to the other graphs too, and the
+    graph that was captured first need not be the one that is replayed first."""
+    run, want = _shared_tiles(2560, 4096)
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    if warm:
+        with torch.cuda.stream(stream):
+            run()
+        stream.synchronize()
+    with torch.cuda.stream(stream):
+        # its scratch is free again, and may be anybody's, when the others are captured
+        spoil, _ = _captured(lambda: torch.full((1 << 17,), 7, dtype=torch.int32, device="cuda").sum(), stream)
+        graphs = [_captured(run, stream, spoil.pool()) for _ in range(2)]
+    torch.cuda.synchronize()
+    for at in (None, 1, None, 0, None, 1, 1, 0, None, None, 0):
+        if at is None:
+            spoil.replay()
+            continue
+        graph, y = graphs[at]
+        y.fill_(float("nan"))
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, want)
+
+
+def test_graphs_of_one_stream_side_by_side():
+    run, want = _shared_tiles(256, 2048)      # (few CTAs: two graphs fit on the GPU at once)
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        run()
+        stream.synchronize()
+        pairs = [_captured(lambda: [run() for _ in range(50)], stream) for _ in range(2)]
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for _, ys in pairs:
+            for y in ys:
+                y.fill_(float("nan"))
+        sides = [torch.cuda.Stream() for _ in pairs]
+        for (graph, _), s in zip(pairs, sides):
+            s.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(s):
+                graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(y, want) for _, ys in pairs for y in ys)
+
+
+def test_counters_of_many_streams_and_captures(monkeypatch):
+    from minisglang_rdna4_b200.ops import cuda as K
+
+    monkeypatch.setattr(K, "_STREAM_COUNTERS", {})
+    monkeypatch.setattr(K, "_CAPTURE_COUNTERS", {})
+    at = [0, 0]
+    monkeypatch.setattr(K, "_stream", lambda: at[0])
+    monkeypatch.setattr(K, "_capture_id", lambda stream: at[1])
+    first = K._stream_counters("cuda", 8)
+    for at[0] in range(1, 3 * K.STREAM_COUNTER_SETS):
+        assert K._stream_counters("cuda", 8) is K._stream_counters("cuda", 9)
+        at[0], keep = 0, at[0]
+        assert K._stream_counters("cuda", 8) is first     # a stream in use keeps its set
+        at[0] = keep
+    assert len(K._STREAM_COUNTERS) == K.STREAM_COUNTER_SETS
+    at[:] = [5, 1]
+    small = K._stream_counters("cuda", 8)
+    large = K._stream_counters("cuda", 10 ** 5)
+    assert large.numel() >= 10 ** 5 and not bool(large.any())
+    assert K._CAPTURE_COUNTERS[("cuda", 5)][1][0] is small        # both stay while their capture goes on
+    at[1] = 2
+    assert K._stream_counters("cuda", 8) is not small and len(K._CAPTURE_COUNTERS[("cuda", 5)][1]) == 1
+
+
 def test_operands_it_does_not_take_are_refused():
     from minisglang_rdna4_b200.ops import cuda as K
     from minisglang_rdna4_b200.ops._lib import lib
