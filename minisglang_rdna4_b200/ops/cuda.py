@@ -707,11 +707,13 @@ class SplitPartial:
 # unreduced. Engines that need verify rows and decode rows on one GEMM code path switch it off.
 SPLIT_K_DECODE = not ENV.DISABLE_SPLIT_K_DECODE.value
 _PENDING_PLANES = False
+PLANES_MOST_COLUMNS = 8192     # widest row of the norm that sums planes (csrc/elementwise.cu, kMaxPlanesRow)
 
 
 def set_next_gemm_planes(on: bool = True) -> None:
-    """Ask the next GEMM call of this thread (M <= 256) to return a ``SplitPartial`` when the
-    split-K plan of its (N, K) has more than one range. Consumed by exactly one call."""
+    """Ask the next GEMM call of this thread to return its K ranges as a ``SplitPartial``: products of up to 128 rows that
+    ``csrc/gemm_stream.cu`` takes and N <= ``PLANES_MOST_COLUMNS``; else those of up to 256 rows whose split-K plan has more
+    than one range. Consumed by exactly one call."""
     global _PENDING_PLANES
     _PENDING_PLANES = on
 
@@ -837,6 +839,7 @@ def _gemm(kind, a, b, n, k, out_dtype, a_scale=None, b_scale=None, bias=None, sf
         return out
     global _PENDING_PLANES
     want_planes, _PENDING_PLANES = _PENDING_PLANES, False
+    want_planes = want_planes and n <= PLANES_MOST_COLUMNS
     if (0 < m <= 128 and bn == 0 and not max_ctas and not SPLIT_K and _stream_pays(m, b.nbytes, want_planes)
             and (few or _decode_step())):
         return _gemm_stream(kind, a, b, m, n, k, out_dtype, a_scale, b_scale, bias, sf_atoms, want_planes)

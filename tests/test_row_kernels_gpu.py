@@ -49,6 +49,40 @@ def test_norm_widths(hidden, planes):
             assert float(((got.double() - want).abs() / want.abs().clamp_min(1e-6)).max()) <= 2.0 ** -8 * 1.01
 
 
+# the widest row whose norm sums planes, and wider ones
+@pytest.mark.parametrize("hidden", [8192, 8200, 12288, 16384])
+@pytest.mark.parametrize("rows", [1, 64, 128, 200])
+@pytest.mark.parametrize("quant", [False, True])
+def test_projection_and_norm_of_a_decode_step(hidden, rows, quant):
+    """A row-parallel projection hands the norm behind it a sum that it can take, at every width a model may have."""
+    from minisglang_rdna4_b200.core import Batch, Context, set_global_ctx
+    from minisglang_rdna4_b200.layers.linear import RowParallelLinear
+    from minisglang_rdna4_b200.layers.norm import RMSNorm
+    from minisglang_rdna4_b200.parallel.comm import get_comm
+    from minisglang_rdna4_b200.parallel.info import set_tp_info
+
+    k = 512
+    set_tp_info(0, 1)
+    proj, norm = RowParallelLinear(k, hidden, torch.bfloat16, "cuda"), RMSNorm(hidden, 1e-6, torch.bfloat16, "cuda")
+    proj.weight, norm.weight = _rand(hidden, k, seed=1), _rand(hidden, seed=2)
+    x, res = _rand(rows, k, seed=3), _rand(rows, hidden, seed=4)
+    get_comm().split_k_ok = True
+    ctx = Context(page_size=16)
+    set_global_ctx(ctx)
+    with ctx.forward_batch(Batch(reqs=[], phase="decode")):
+        got, new = norm.forward_fused(proj.forward(x), res.clone(), partial=True, quant=quant)
+    y = x.double() @ proj.weight.double().t()
+    # the projection and the sum with the residual are rounded to 16 bits each: half a step of eight significant bits, at most
+    # 2^-8 of either; and fp32 sums of k products
+    want = y + res.double()
+    assert float(((new.double() - want).abs() - 2.0 ** -8 * (y.abs() + want.abs()) * 1.01).max()) <= 2.0 ** -12
+    norm16 = (new.double() * torch.rsqrt(new.double().square().mean(-1, keepdim=True) + 1e-6) * norm.weight.double())
+    if quant:
+        _same_rows8((got.q, got.scale), norm16.to(torch.bfloat16))
+    else:
+        assert float(((got.double() - norm16).abs() / norm16.abs().clamp_min(1e-6)).max()) <= 2.0 ** -8 * 1.01
+
+
 def test_a_norm_does_not_depend_on_the_rows_around():
     from minisglang_rdna4_b200.ops import cuda as K
 
