@@ -10,6 +10,7 @@
 // set. Semantics follow python/minisgl/engine/sample.py:108-142 (min-p floor, then top-k, then
 // top-p over the surviving mass, renormalise, draw).
 #include "common.cuh"
+#include "ptx.cuh"
 
 #include <cooperative_groups.h>
 
@@ -33,6 +34,9 @@ __device__ __forceinline__ ArgMax better(ArgMax a, ArgMax b) {
 // flight: 151936 columns, one CTA per row -> this, us: 1 row 15.0 -> 4.1, 64 rows 16.2 -> 10.8.
 __global__ void __launch_bounds__(512) argmax_kernel(const float* __restrict__ logits, int32_t* __restrict__ out,
                                                      int vocab, long long stride) {
+  // A CTA's shared memory may be written by the others once it runs: each says so here, and waits for the others to have
+  // said so in front of its store. The scan of the row lies in between.
+  if (gridDim.x > 1) ptx::cluster_arrive_all();
   pdl_enter();
   __shared__ ArgMax red[16];
   __shared__ ArgMax all[kArgmaxCtas];
@@ -78,8 +82,10 @@ __global__ void __launch_bounds__(512) argmax_kernel(const float* __restrict__ l
   }
   if (gridDim.x > 1) {
     cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    ptx::cluster_wait_all();
     if (threadIdx.x == 0) *cluster.map_shared_rank(all + blockIdx.x, 0) = best;
-    cluster.sync();
+    __syncwarp();
+    ptx::cluster_sync_all();
     if (blockIdx.x != 0) return;
     if (warp == 0) {
       best = lane < (int)gridDim.x ? all[lane] : ArgMax{-INFINITY, 0x7fffffff};

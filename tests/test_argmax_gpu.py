@@ -27,3 +27,22 @@ def test_argmax_of_shares(vocab, rows):
     wide = torch.full((rows, vocab + 3), 1000.0, device="cuda")
     wide[:, :vocab] = x
     assert torch.equal(K.argmax(wide[:, :vocab]).long(), torch.where(torch.isinf(x.amax(-1)), 0, x.argmax(-1)))
+
+
+def test_beside_other_work():
+    """CTAs of a cluster that start far apart, behind and beside kernels that hold most of the GPU: the one that takes the others'
+    results may be the last to start, and the others have next to nothing to scan."""
+    from minisglang_rdna4_b200.ops import cuda as K
+
+    x = _rand(37, 16384, dtype=torch.float32)
+    want = x.argmax(-1)
+    busy = _rand(4096, 4096)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    got = []
+    for _ in range(50):
+        with torch.cuda.stream(side):
+            busy = (busy @ busy).clamp(-1, 1)
+        got += [K.argmax(x) for _ in range(8)]
+    torch.cuda.synchronize()
+    assert all(torch.equal(g.long(), want) for g in got)
