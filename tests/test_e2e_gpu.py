@@ -49,6 +49,30 @@ def test_generate_graph_matches_eager(quant, kv):
     assert outs["chunked"] == outs["eager"]
 
 
+@pytest.mark.parametrize("quant,kv", [(None, "bf16"), ("mxfp4", "fp8")])
+def test_graphs_of_many_sizes_match_eager(quant, kv):
+    """One request before any larger graph has run, many, one again, and each time the tokens of eager steps: a graph starts from
+    nothing that another one leaves behind."""
+    from minisglang_rdna4_b200 import SamplingParams
+    from minisglang_rdna4_b200.llm import LLM
+    from minisglang_rdna4_b200.ops import cuda as K
+
+    g = torch.Generator().manual_seed(11)
+    prompts = [torch.randint(0, 2048, (5 + i % 23,), generator=g).tolist() for i in range(90)]
+    sp = SamplingParams(temperature=0.0, max_tokens=6, ignore_eos=True)
+    outs = {}
+    for name, kw in (("graph", dict()), ("eager", dict(cuda_graph_max_bs=-1))):
+        llm = LLM(model_config=_cfg(), use_dummy_weight=True, quantization=quant, kv_cache_dtype=kv,
+                  device="cuda", page_size=16, max_running_req=96, num_page_override=512, seed=0, **kw)
+        runs = [prompts[:1], prompts, prompts[1:2], prompts[:40], prompts[2:3], prompts]
+        outs[name] = [[o.token_ids for o in llm.generate(r, sp)] for r in runs]
+        runner = llm.engine.graph_runner
+        assert (runner is not None and runner.replays > 0) == (name == "graph")
+        assert K.gemm_status() == 0 and K.attn_status() == 0
+        llm.shutdown()
+    assert outs["graph"] == outs["eager"]
+
+
 def test_bf16_engine_tracks_fp32_oracle():
     """Same random weights on the CPU fp32 oracle path: the first generated tokens agree for
     most prompts (bf16 rounding may flip near-ties later in a sequence)."""
