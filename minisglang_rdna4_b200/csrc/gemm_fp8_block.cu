@@ -12,20 +12,22 @@
 // The scales change every 128 elements of K and are arbitrary fp32 numbers, so they cannot ride
 // on the block-scaled MMA kinds (those take power-of-two UE8M0 scales). Instead every K block
 // (= one pipeline stage, four tcgen05.mma kind::f8f6f4 of K = 32) is accumulated on its own
-// into one of four 128-column tensor-memory buffers; the eight promotion warps pull a finished
-// block out with tcgen05.ld, multiply by the block's scale product and add it to a 64-float
-// register accumulator per row and half while the tensor core already works on the next blocks in the
+// into one of four 128-column tensor-memory buffers; the four promotion warps pull a finished
+// block out with tcgen05.ld, multiply by the block's scale product and add it to a 128-float
+// register accumulator per row while the tensor core already works on the next blocks in the
 // other buffers. Every row's sum runs over K in ascending order and does not depend on M.
 //
 // Structure as in gemm_tcgen05.cu: persistent CTAs, warp 0 = TMA producer, warp 1 = MMA issuer
-// and tensor-memory owner, warps 2-9 = promotion + store. All waits are bounded.
+// and tensor-memory owner, warps 2-5 = promotion + store. All waits are bounded.
 //
 // Bound of many rows: what an SM takes in from L2, 32 KB for each K block of a tile (with the MMAs, the promotion and the stores all
 // left out a block still takes 0.49 us, 65 GB/s an SM). On top of that came the stores: a lane wrote 16 bytes of its own row at a time,
 // a quarter of the time of the first product and 30 % of the second. A warp now packs its 32 x 64 results into shared memory and
-// leaves them to one TMA store, whose end it waits for before the next tile's. B200, 4480 tokens with 8 of 128 experts, us:
-// N 1536, K 2048 326 -> 270, N 2048, K 768 181 -> 135; 1024 tokens, the whole layer 236 -> 211. (Eight promotion warps in the place of four and
-// four partial buffers in the place of two changed nothing by themselves; they make room for the stores.)
+// leaves them to one TMA store, whose end it waits for before the next tile's. Eight promotion warps of 64 columns each were 2 to 4 %
+// slower than four (4096 x 4096, 100 rows 17.1 -> 16.5 us; 24576 x 4096, 1024 rows 159 -> 154), two partial buffers with a sixth stage up to 5 %
+// slower than four with five for many rows.
+// B200, us, stores of the lanes -> this: 24576 x 4096, 4096 rows 647 -> 593, 1024 rows 173 -> 154, 100 rows 33.6 -> 31.9; 1536 x 2048, 4096
+// rows 29.2 -> 25.1; 4096 x 4096, 128 rows 16.5 -> 16.6, 16 rows 15.4 -> 16.1 (a store's end is waited for).
 #include "common.cuh"
 #include "ptx.cuh"
 
@@ -41,14 +43,13 @@ int msgl_b_static_level();   // gemm_tcgen05.cu: level set by msgl_gemm_static_w
 namespace {
 
 constexpr int BM = 128, BN = 128, BK = 128;
-constexpr int kThreads = 320;      // TMA, MMA, eight promotion warps
-constexpr int kFewThreads = 192;   // four promotion warps
+constexpr int kThreads = 192;      // TMA, MMA, four promotion warps
 constexpr int PARTS = 4;           // partial buffers
 constexpr int STAGES = 5;
 constexpr int A_BYTES = BM * BK, B_BYTES = BN * BK;
 constexpr int off_a = 0;
 constexpr int off_b = off_a + STAGES * A_BYTES;
-constexpr int PATCH_BYTES = 32 * 128;   // a promotion warp's results: 32 rows of 64 16-bit columns
+constexpr int PATCH_BYTES = 32 * 128;   // half of a promotion warp's results: 32 rows of 64 16-bit columns
 constexpr int off_patch = off_b + STAGES * B_BYTES;
 constexpr int off_bar = off_patch + 8 * PATCH_BYTES;
 constexpr int n_bars = 2 * STAGES + 2 * PARTS;  // full / empty per stage, pfull / pempty per partial buffer
@@ -95,7 +96,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
     }
     for (int s = 0; s < PARTS; ++s) {
       mbar_init(pfull_bar(s), 1);
-      mbar_init(pempty_bar(s), 8);
+      mbar_init(pempty_bar(s), 4);
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -177,11 +178,9 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       }
     }
   } else {
-    // ------------------------------------------------------------------ promotion + store (warps 2..9)
-    constexpr int W = BN / 2;
-    const int q = warp & 3;                  // tensor-memory lane quarter this warp may read
-    const int half = (warp - 2) >> 2;        // which 64 of the tile's 128 columns
-    const bool pairs = args.k_blocks % 2 == 0;   // row scales can be read two at a time
+    // ------------------------------------------------------------------ promotion + store (warps 2..5)
+    constexpr int W = BN / 2;   // columns that are read at once
+    const int q = warp & 3;     // tensor-memory lane quarter this warp may read
     int pb = 0;
     uint32_t pphase = 0;
     bool ok = true;
@@ -196,83 +195,82 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       const bool row_ok = row < args.M;
       const float* as_row = args.a_scale + (size_t)(row_ok ? row : 0) * args.k_blocks;
       const float* ws_row = args.w_scale + ((size_t)expert * args.n_tiles + n_tile) * args.k_blocks;
-      float as_odd = 0.f;
-      auto scale_of = [&](int kb) {   // asked for in ascending order
-        float a;
-        if (!pairs) {
-          a = __ldg(as_row + kb);
-        } else if ((kb & 1) == 0) {
-          const float2 two = __ldg(reinterpret_cast<const float2*>(as_row + kb));
-          a = two.x;
-          as_odd = two.y;
-        } else {
-          a = as_odd;
-        }
-        return row_ok ? a * __ldg(ws_row + kb) : 0.f;
-      };
-      float acc[W];
+      float acc[2][W];
 #pragma unroll
-      for (int e = 0; e < W; ++e) acc[e] = 0.f;
-      float s_next = scale_of(0);
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int e = 0; e < W; ++e) acc[h][e] = 0.f;
+      float as_next = row_ok ? __ldg(as_row) : 0.f, ws_next = row_ok ? __ldg(ws_row) : 0.f;
       for (int kb = 0; kb < args.k_blocks; ++kb) {
-        const float s = s_next;
-        if (kb + 1 < args.k_blocks) s_next = scale_of(kb + 1);
+        const float s = as_next * ws_next;
+        if (kb + 1 < args.k_blocks && row_ok) {
+          as_next = __ldg(as_row + kb + 1);
+          ws_next = __ldg(ws_row + kb + 1);
+        }
         if (!mbar_wait(pfull_bar(pb), pphase, abort_flag, args.status, 124)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(pb * BN + half * W);
-        uint32_t r0[32], r1[32];
-        tmem_ld_32x32b_x32(t_addr, r0);
-        tmem_ld_32x32b_x32(t_addr + 32, r1);
-        tmem_ld_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(pempty_bar(pb));
+        const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(pb * BN);
 #pragma unroll
-        for (int e = 0; e < 32; ++e) {
-          acc[e] = fmaf(__uint_as_float(r0[e]), s, acc[e]);
-          acc[32 + e] = fmaf(__uint_as_float(r1[e]), s, acc[32 + e]);
+        for (int h = 0; h < 2; ++h) {
+          uint32_t r0[32], r1[32];
+          tmem_ld_32x32b_x32(t_addr + h * W, r0);
+          tmem_ld_32x32b_x32(t_addr + h * W + 32, r1);
+          tmem_ld_wait();
+          if (h == 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(pempty_bar(pb));
+          }
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            acc[h][e] = fmaf(__uint_as_float(r0[e]), s, acc[h][e]);
+            acc[h][32 + e] = fmaf(__uint_as_float(r1[e]), s, acc[h][32 + e]);
+          }
         }
         if (++pb == PARTS) { pb = 0; pphase ^= 1u; }
       }
       if (!ok) break;
-      const int colbase = n_tile * BN + half * W;
-      auto pack = [&](int i) {   // columns 2i and 2i + 1
-        if (args.out_dtype == MSGL_BF16) {
-          __nv_bfloat162 v = __floats2bfloat162_rn(acc[2 * i], acc[2 * i + 1]);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int colbase = n_tile * BN + h * W;
+        auto pack = [&](int i) {   // columns 2i and 2i + 1
+          if (args.out_dtype == MSGL_BF16) {
+            __nv_bfloat162 v = __floats2bfloat162_rn(acc[h][2 * i], acc[h][2 * i + 1]);
+            return *reinterpret_cast<uint32_t*>(&v);
+          }
+          __half2 v = __floats2half2_rn(acc[h][2 * i], acc[h][2 * i + 1]);
           return *reinterpret_cast<uint32_t*>(&v);
-        }
-        __half2 v = __floats2half2_rn(acc[2 * i], acc[2 * i + 1]);
-        return *reinterpret_cast<uint32_t*>(&v);
-      };
-      if (args.tma_out) {
-        uint8_t* const patch = smem + off_patch + (warp - 2) * PATCH_BYTES;
-        if (lane == 0) bulk_wait_group_read<0>();   // the tile before this one has left the patch
-        __syncwarp();
+        };
+        if (args.tma_out) {
+          uint8_t* const patch = smem + off_patch + (q * 2 + h) * PATCH_BYTES;
+          if (h == 0 && lane == 0) bulk_wait_group_read<0>();   // the tile before this one has left the patch
+          __syncwarp();
 #pragma unroll
-        for (int u = 0; u < 8; ++u)   // 128-byte swizzle: 16-byte unit u of row r lives at unit u ^ (r & 7)
-          *reinterpret_cast<uint4*>(patch + lane * 128 + ((u ^ (lane & 7)) << 4)) =
-              make_uint4(pack(u * 4), pack(u * 4 + 1), pack(u * 4 + 2), pack(u * 4 + 3));
-        fence_proxy_async();
-        __syncwarp();
-        const int row0 = m_tile * BM + q * 32;
-        if (lane == 0 && row0 < args.M && colbase < args.N) {
-          tma_store_2d(&tma_c, s_base + off_patch + (warp - 2) * PATCH_BYTES, colbase, row0);
-          bulk_commit_group();
-        }
-      } else if (row_ok) {
-        if (args.out_dtype == MSGL_F32) {
-          float* crow = reinterpret_cast<float*>(args.c) + (size_t)row * args.ldc + colbase;
+          for (int u = 0; u < 8; ++u)   // 128-byte swizzle: 16-byte unit u of row r lives at unit u ^ (r & 7)
+            *reinterpret_cast<uint4*>(patch + lane * 128 + ((u ^ (lane & 7)) << 4)) =
+                make_uint4(pack(u * 4), pack(u * 4 + 1), pack(u * 4 + 2), pack(u * 4 + 3));
+          fence_proxy_async();
+          __syncwarp();
+          const int row0 = m_tile * BM + q * 32;
+          if (lane == 0 && row0 < args.M && colbase < args.N) {
+            tma_store_2d(&tma_c, s_base + off_patch + (q * 2 + h) * PATCH_BYTES, colbase, row0);
+            bulk_commit_group();
+          }
+        } else if (row_ok) {
+          if (args.out_dtype == MSGL_F32) {
+            float* crow = reinterpret_cast<float*>(args.c) + (size_t)row * args.ldc + colbase;
 #pragma unroll
-          for (int g = 0; g < W / 4; ++g)
-            if (colbase + g * 4 < args.N)
-              *reinterpret_cast<float4*>(crow + g * 4) =
-                  make_float4(acc[g * 4], acc[g * 4 + 1], acc[g * 4 + 2], acc[g * 4 + 3]);
-        } else {
-          uint16_t* crow = reinterpret_cast<uint16_t*>(args.c) + (size_t)row * args.ldc + colbase;
+            for (int g = 0; g < W / 4; ++g)
+              if (colbase + g * 4 < args.N)
+                *reinterpret_cast<float4*>(crow + g * 4) =
+                    make_float4(acc[h][g * 4], acc[h][g * 4 + 1], acc[h][g * 4 + 2], acc[h][g * 4 + 3]);
+          } else {
+            uint16_t* crow = reinterpret_cast<uint16_t*>(args.c) + (size_t)row * args.ldc + colbase;
 #pragma unroll
-          for (int g = 0; g < W / 8; ++g)
-            if (colbase + g * 8 < args.N)
-              *reinterpret_cast<uint4*>(crow + g * 8) = make_uint4(pack(g * 4), pack(g * 4 + 1), pack(g * 4 + 2), pack(g * 4 + 3));
+            for (int g = 0; g < W / 8; ++g)
+              if (colbase + g * 8 < args.N)
+                *reinterpret_cast<uint4*>(crow + g * 8) = make_uint4(pack(g * 4), pack(g * 4 + 1), pack(g * 4 + 2), pack(g * 4 + 3));
+          }
         }
       }
     }
@@ -374,7 +372,7 @@ struct FewArgs {
 };
 
 template <int NB, bool GLU>
-__global__ void __launch_bounds__(kFewThreads, 1)
+__global__ void __launch_bounds__(kThreads, 1)
 gemm_fp8_block_few_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_constant__ CUtensorMap tma_x, const FewArgs args) {
   using C = FewCfg<NB>;
   constexpr int STAGES_ = C::STAGES;
@@ -710,7 +708,7 @@ int launch_few(const CUtensorMap& mw, const CUtensorMap& mx, const FewArgs& args
   static const cudaError_t configured =
       cudaFuncSetAttribute(gemm_fp8_block_few_kernel<NB, GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   cudaError_t e = configured;
-  if (e == cudaSuccess) e = msgl_launch(gemm_fp8_block_few_kernel<NB, GLU>, dim3(ctas), dim3(kFewThreads), smem, stream, mw, mx, args);
+  if (e == cudaSuccess) e = msgl_launch(gemm_fp8_block_few_kernel<NB, GLU>, dim3(ctas), dim3(kThreads), smem, stream, mw, mx, args);
   if (e != cudaSuccess) { msgl_set_error("gemm_fp8_block_few", e); return MSGL_CUDA_ERROR; }
   return MSGL_OK;
 }

@@ -54,6 +54,28 @@ def test_against_64_bits(counts, n, k, block, dtype):
     assert K.gemm_fp8_block_status() == 0
 
 
+# an even and an odd number of K blocks, one tile and several of a CTA
+@pytest.mark.parametrize("m,n,k", [(5, 256, 512), (130, 1000, 640), (700, 8192, 256)])
+def test_dense_scales_at_any_address(m, n, k):
+    """Scales are single fp32 numbers: a view that begins in the middle of 8 or 16 bytes is read as any other."""
+    from minisglang_rdna4_b200.ops import cuda as K
+
+    g = torch.Generator("cuda")
+    g.manual_seed(m)
+    pad = -n % 128
+    w, ws = _blocks8(torch.randn(1, n + pad, k, generator=g, device="cuda") * 0.02)
+    w, ws = w[0, :n].contiguous(), ws[0]
+    xq, xs = K.per_group_quant_fp8(torch.randn(m, k, generator=g, device="cuda").bfloat16(), 128)
+    want = K.gemm_fp8_block(xq, xs, w, ws)
+    full = (xq.double().view(m, -1, 128) * xs.double()[..., None]).view(m, k) @ _wide(
+        torch.nn.functional.pad(w.view(torch.uint8), (0, 0, 0, pad)).view(torch.float8_e4m3fn)[None], ws[None])[0, :n].t()
+    assert float((want.double() - full).norm() / full.norm()) < 2.0 ** -9 + 1e-5
+    for off in (1, 2, 3):
+        at = lambda t: torch.cat([t.new_zeros(off), t.reshape(-1)])[off:].view(t.shape)  # noqa: E731
+        assert at(xs).data_ptr() % 16 == 4 * off
+        assert torch.equal(K.gemm_fp8_block(xq, at(xs), w, at(ws)), want)
+
+
 def test_a_layer_in_both_forms():
     from minisglang_rdna4_b200.ops import moe_kernels as MK
 
