@@ -31,14 +31,15 @@ __device__ __forceinline__ ArgMax better(ArgMax a, ArgMax b) {
 }
 
 // A cluster of gridDim.x CTAs per row, each with a contiguous share of it. Bound: for few rows the loads that one SM keeps in
-// flight: 151936 columns, one CTA per row -> this, us: 1 row 15.0 -> 4.1, 64 rows 16.2 -> 10.8.
-__global__ void __launch_bounds__(512) argmax_kernel(const float* __restrict__ logits, int32_t* __restrict__ out,
+// flight. argmax_plan has the times.
+template <int THREADS, int CTAS>
+__global__ void __launch_bounds__(THREADS, CTAS) argmax_kernel(const float* __restrict__ logits, int32_t* __restrict__ out,
                                                      int vocab, long long stride) {
   // A CTA's shared memory may be written by the others once it runs: each says so here, and waits for the others to have
   // said so in front of its store. The scan of the row lies in between.
   if (gridDim.x > 1) ptx::cluster_arrive_all();
   pdl_enter();
-  __shared__ ArgMax red[16];
+  __shared__ ArgMax red[THREADS / 32];
   __shared__ ArgMax all[kArgmaxCtas];
   const float* row = logits + (size_t)blockIdx.y * stride;
   ArgMax best{-INFINITY, 0x7fffffff};
@@ -209,25 +210,58 @@ __global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ 
 
 }  // namespace
 
+namespace {
+
+struct ArgMaxPlan {
+  int ctas, threads;   // of a row's cluster, of a CTA
+  bool two;            // the form of which two CTAs of 1024 threads fit on an SM
+};
+
+// A share of less than 2048 values is one round of loads: nothing to split. Clusters of CTAs that do not all fit at once start in
+// rounds, so a row has as many CTAs as keep the whole within the SMs; of wide rows up to four CTAs of 512 threads on an SM, whose loads
+// make up for that. Up to two rows for each SM, one CTA a row of the form that fits twice.
+// B200, us, 1024 threads a row -> this: 151936 columns, 1 row 13.7 -> 3.6, 16 14.2 -> 4.9, 48 14.3 -> 6.7, 64 14.4 -> 7.8 (clusters of 8: 10.5), 100
+// 14.4 -> 9.9, 150 24.1 -> 19.6, 256 28.9 -> 27.2 (without the form for two: 34); 16384 columns, 1 row 2.6 -> 2.2, 64 2.9 -> 2.8 (clusters of 8: 5.4),
+// 256 4.2 -> 4.1; 32000, 64 4.3 -> 3.5, 256 6.1 -> 6.2.
+ArgMaxPlan argmax_plan(int rows, int vocab) {
+  constexpr int sms = 148;
+  const bool two = rows > sms && rows <= 2 * sms;
+  if (vocab < kArgmaxCtas * 2048) return {1, 512, two};
+  if (vocab < 65536) {
+    if (rows <= sms / 2) return {rows <= sms / 8 ? 8 : rows <= sms / 4 ? 4 : 2, 512, false};
+    return {1, 512, two};
+  }
+  if (rows <= 50) return {8, 512, false};
+  if (rows <= sms / 2) return {2, 1024, true};
+  if (rows <= sms) return {4, 512, false};
+  if (rows <= sms * 3 / 2) return {2, 512, false};
+  return {1, two ? 1024 : 512, two};
+}
+
+}  // namespace
+
 MSGL_API int msgl_argmax(const void* logits, void* out, int rows, int vocab, long long stride, cudaStream_t stream) {
   if (rows == 0) return MSGL_OK;
-  // A share of less than 2048 values is one round of loads: nothing to split. Nor is there where the rows alone give every SM
-  // four CTAs (256 rows in clusters of 8: 36 us, against 31 unsplit). Rows ride in the grid's y (65535 a launch).
-  int ctas = vocab >= kArgmaxCtas * 2048 ? kArgmaxCtas : 1;
-  while (ctas > 1 && (long long)rows * ctas > 4 * 148) ctas /= 2;
+  const ArgMaxPlan plan = argmax_plan(rows, vocab);
+  auto* const kernel = plan.two ? argmax_kernel<1024, 2> : argmax_kernel<512, 3>;
   for (int r0 = 0; r0 < rows; r0 += 65535) {
     cudaLaunchAttribute attr[2] = {};
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim = {(unsigned)ctas, 1, 1};
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    int attrs = 0;
+    if (msgl_pdl_enabled()) {
+      attr[attrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[attrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (plan.ctas > 1) {
+      attr[attrs].id = cudaLaunchAttributeClusterDimension;
+      attr[attrs++].val.clusterDim = {(unsigned)plan.ctas, 1, 1};
+    }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ctas, rows - r0 < 65535 ? rows - r0 : 65535);
-    cfg.blockDim = dim3(512);
+    cfg.gridDim = dim3(plan.ctas, rows - r0 < 65535 ? rows - r0 : 65535);
+    cfg.blockDim = dim3(plan.threads);
     cfg.stream = stream;
     cfg.attrs = attr;
-    cfg.numAttrs = msgl_pdl_enabled() ? 2 : 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, argmax_kernel, (const float*)logits + (size_t)r0 * stride, (int32_t*)out + r0,
+    cfg.numAttrs = attrs;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, (const float*)logits + (size_t)r0 * stride, (int32_t*)out + r0,
                                              vocab, stride);
     if (e != cudaSuccess) { msgl_set_error("argmax", e); return MSGL_CUDA_ERROR; }
   }

@@ -29,6 +29,18 @@ def test_argmax_of_shares(vocab, rows):
     assert torch.equal(K.argmax(wide[:, :vocab]).long(), torch.where(torch.isinf(x.amax(-1)), 0, x.argmax(-1)))
 
 
+# on both sides of every line of the plan
+@pytest.mark.parametrize("vocab,rows", [(v, r) for v in (16383, 16384, 65535, 65536) for r in
+                                        (18, 19, 37, 38, 50, 51, 74, 75, 148, 149, 222, 223, 296, 297)])
+def test_argmax_of_any_number_of_rows(vocab, rows):
+    from minisglang_rdna4_b200.ops import cuda as K
+
+    x = _rand(rows, vocab, dtype=torch.float32)
+    at = torch.arange(rows, device="cuda")
+    x[at, (at * 7919) % vocab] = 60.0
+    assert torch.equal(K.argmax(x).long(), (at * 7919) % vocab)
+
+
 def test_beside_other_work():
     """CTAs of a cluster that start far apart, behind and beside kernels that hold most of the GPU: the one that takes the others'
     results may be the last to start, and the others have next to nothing to scan."""
