@@ -68,10 +68,12 @@ MSGL_API int msgl_embedding(const void* ids, const void* w, void* out, int rows,
 // Bound: HBM for many rows, one memory round trip for few. All loads of a row (x, residual, weight; of
 // planes four at a time) are issued before the first store: with the residual's store between two
 // vectors' loads each of up to eight vectors cost a round trip of its own. Threads and vectors a thread are
-// chosen by the width alone (never by the row count: the order of the sum, and with it a row's bits,
-// would follow), two vectors a thread, so that a decode step's few rows have all their bytes under way too.
+// chosen by the width and the form alone (never by the row count: the order of the sum, and with it a row's bits,
+// would follow): two vectors a thread, so that a decode step's few rows have all their bytes under way too, four above 4096 columns,
+// where 512 and more threads a row leave too few rows on an SM, and without a residual, which halves the bytes of a row, above 2560.
 // B200, us, with the residual and e4m3 out, before -> after: 1 x 2560 3.9 -> 2.7, 64 x 4096 4.7 -> 3.1, 8190 x 2560 31.5 -> 30.3,
-// 8192 x 8192 120 -> 110 (4.3 TB/s); 5 planes of 64 x 4096 7.6 -> 4.5, 3 of 32 x 8192 11.9 -> 4.9.
+// 8190 x 8192 120 -> 107, 8190 x 12288 255 -> 200, 16 bits out 256 -> 140; without a residual 8190 x 8192 76 -> 64 (two vectors: 82), 8190 x 12288
+// 117 -> 98 (157), 8190 x 4096 32.0 -> 32.7 (35.1), 16 x 4096 2.8 -> 2.0; 5 planes of 64 x 4096 7.6 -> 4.5, 3 of 32 x 8192 11.9 -> 4.9.
 // ------------------------------------------------------------------------------------------
 template <typename T, bool ADD, bool QUANT, int VPT, int MAXT, bool PLANES = false>
 __global__ void __launch_bounds__(MAXT) rms_norm_kernel(const T* __restrict__ x, T* __restrict__ residual,
@@ -192,7 +194,7 @@ static void launch_rms_vpt(const void* x, int planes, void* residual, const void
 #define RMS_LAUNCH(A, Q, P)                                                                                                   \
   msgl_launch(rms_norm_kernel<T, A, Q, VPT, MAXT, P>, dim3(rows), dim3(threads), 0, s, (const T*)x, (T*)residual, (const T*)w, \
               (T*)out, (uint8_t*)out_q, (float*)out_scale, hidden, eps, off, planes, stride)
-  if constexpr (MAXT * VPT * 8 <= kMaxPlanesRow) {
+  if constexpr (MAXT * VPT * 8 <= kMaxPlanesRow && VPT < 4) {
     if (planes > 0) {
       if (quant) RMS_LAUNCH(true, true, true);
       else RMS_LAUNCH(true, false, true);
@@ -211,10 +213,15 @@ static int launch_rms(const void* x, int planes, void* residual, const void* w, 
                       int hidden, float eps, int plus_one, cudaStream_t s) {
   const float off = plus_one ? 1.f : 0.f;
   const int vecs = hidden / 8;
-  if (vecs <= 128) launch_rms_vpt<T, 1, 128>(x, planes, residual, w, out, out_q, out_scale, rows, hidden, eps, off, s);
-  else if (vecs <= 512) launch_rms_vpt<T, 2, 256>(x, planes, residual, w, out, out_q, out_scale, rows, hidden, eps, off, s);
-  else if (vecs <= 1024) launch_rms_vpt<T, 2, 512>(x, planes, residual, w, out, out_q, out_scale, rows, hidden, eps, off, s);
-  else launch_rms_vpt<T, 2, 1024>(x, planes, residual, w, out, out_q, out_scale, rows, hidden, eps, off, s);
+  const bool plain = residual == nullptr && out_q == nullptr;
+#define RMS(V, TH) launch_rms_vpt<T, V, TH>(x, planes, residual, w, out, out_q, out_scale, rows, hidden, eps, off, s)
+  if (vecs <= 128) RMS(1, 128);
+  else if (vecs <= 512 && !(plain && vecs > 320)) RMS(2, 256);
+  else if (vecs <= 512) RMS(4, 128);
+  else if (planes > 0) RMS(2, 512);   // (whose loads of four planes are registers enough)
+  else if (vecs <= 1024) RMS(4, 256);
+  else RMS(4, 512);
+#undef RMS
   MSGL_CHECK_LAUNCH("rms_norm");
   return MSGL_OK;
 }
@@ -351,7 +358,7 @@ __global__ void __launch_bounds__(THREADS) act_mul_quant_kernel(const T* __restr
 template <typename T, int KIND>
 static int launch_act_quant(const void* x, void* out_q, void* out_scale, int rows, int inter, cudaStream_t s) {
   // the widest block that has a few vectors for every thread; a decode step's few rows take twice the threads, which have
-  // more of a row under way at once
+  // more of a row under way at once (8190 x 1408: 11.3 us with 128 threads, 13.3 with 256; 1 x 1408 1.6 and 1.5)
   const int vecs = inter / 8;
 #define ACT_LAUNCH(V, TH) \
   msgl_launch(act_mul_quant_kernel<T, V, TH, KIND>, dim3(rows), dim3(TH), 0, s, (const T*)x, (uint8_t*)out_q, (float*)out_scale, inter)
@@ -366,6 +373,7 @@ static int launch_act_quant(const void* x, void* out_q, void* out_scale, int row
   } else {
     const int vpt = (vecs + 255) / 256;
     if (vecs <= 128) ACT_LAUNCH(1, 128);
+    else if (vecs <= 256 && rows > 2048) ACT_LAUNCH(2, 128);
     else if (vpt <= 1) ACT_LAUNCH(1, 256);
     else if (vpt <= 2) ACT_LAUNCH(2, 256);
     else if (vpt <= 3) ACT_LAUNCH(3, 256);
@@ -418,7 +426,8 @@ MSGL_API int msgl_act_and_mul(const void* x, void* out, void* out_q, void* out_s
 // stand-alone activation quantisers: per token (group == hidden) or per `group` elements
 // ------------------------------------------------------------------------------------------
 // A group is one row of up to 16384 elements (a CTA each, VPT 16-byte vectors a thread, read once), or a run of
-// elements of any multiple of 8 (a power of two of lanes each, vectors 16 bytes a lane). B200, us, a warp for each group of any
+// elements of any multiple of 8 (a power of two of lanes each, vectors 16 bytes a lane). Many short rows are runs too: a CTA of one or
+// two warps for each costs more than it reads (8190 x 512 4.2 us against 8.9, 8190 x 1024 6.6 against 9.0; 2397 x 1024 3.5 against 2.9). B200, us, a warp for each group of any
 // length and two passes over it -> now: 1 x 4096 3.7 -> 1.8, 256 x 4096 5.1 -> 2.7, 8192 x 8192 53 -> 38; 16640 x 2048 in groups of 128
 // 51 -> 33.
 template <typename T, int VPT>
@@ -457,26 +466,27 @@ __global__ void __launch_bounds__(512) quant_row_kernel(const T* __restrict__ x,
   }
 }
 
-template <typename T>
-__global__ void quant_group_kernel(const T* __restrict__ x, uint8_t* __restrict__ out_q,
-                                   float* __restrict__ out_scale, int group, int lanes, size_t total_groups) {
+template <typename T, int LANES>
+__global__ void __launch_bounds__(256) quant_group_kernel(const T* __restrict__ x, uint8_t* __restrict__ out_q,
+                                                          float* __restrict__ out_scale, int group, size_t total_groups) {
   pdl_enter();
-  const size_t gidx = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / lanes;
+  const size_t gidx = ((size_t)blockIdx.x * 256 + threadIdx.x) / LANES;
   const bool live = gidx < total_groups;
-  const int lane = threadIdx.x & (lanes - 1);
+  const int lane = threadIdx.x & (LANES - 1);
   const T* src = x + gidx * group;
   float amax = 0.f;
-  for (int i = lane * 8; live && i < group; i += lanes * 8) {
+  for (int i = lane * 8; live && i < group; i += LANES * 8) {
     float v[8];
     load8(src + i, v);
 #pragma unroll
     for (int k = 0; k < 8; ++k) amax = fmaxf(amax, fabsf(v[k]));
   }
-  for (int o = lanes >> 1; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+#pragma unroll
+  for (int o = LANES >> 1; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
   if (!live) return;
   const float scale = fmaxf(amax, 1e-8f) / kFp8Max;
   if (lane == 0) out_scale[gidx] = scale;
-  for (int i = lane * 8; i < group; i += lanes * 8) {
+  for (int i = lane * 8; i < group; i += LANES * 8) {
     float v[8];
     load8(src + i, v);
     *reinterpret_cast<uint2*>(out_q + gidx * group + i) = pack8_e4m3(v, scale);
@@ -486,7 +496,8 @@ __global__ void quant_group_kernel(const T* __restrict__ x, uint8_t* __restrict_
 template <typename T>
 static void launch_quant(const void* x, void* out_q, void* out_scale, size_t total, int group, cudaStream_t s) {
   const int vecs = group / 8;
-  if (vecs > 32 && vecs <= 4 * 512) {
+  const bool runs = vecs <= 32 || (vecs <= 64 && total >= 2048) || (vecs <= 128 && total >= 4096);
+  if (!runs && vecs <= 4 * 512) {
     const int vpt = vecs <= 64 ? 1 : vecs <= 1024 ? 2 : 4, threads = ((vecs + vpt - 1) / vpt + 31) / 32 * 32;
 #define QUANT_ROW(V) \
   msgl_launch(quant_row_kernel<T, V>, dim3((unsigned)total), dim3(threads), 0, s, (const T*)x, (uint8_t*)out_q, (float*)out_scale, group)
@@ -496,11 +507,16 @@ static void launch_quant(const void* x, void* out_q, void* out_scale, size_t tot
 #undef QUANT_ROW
     return;
   }
-  int lanes = 1;
-  while (lanes < vecs && lanes < 32) lanes *= 2;
-  const unsigned blocks = (unsigned)((total * lanes + 255) / 256);
-  msgl_launch(quant_group_kernel<T>, dim3(blocks), dim3(256), 0, s, (const T*)x, (uint8_t*)out_q, (float*)out_scale, group, lanes,
-              total);
+#define QUANT_GROUPS(L)                                                                                                            \
+  msgl_launch(quant_group_kernel<T, L>, dim3((unsigned)((total * L + 255) / 256)), dim3(256), 0, s, (const T*)x, (uint8_t*)out_q, \
+              (float*)out_scale, group, total)
+  if (vecs <= 1) QUANT_GROUPS(1);
+  else if (vecs <= 2) QUANT_GROUPS(2);
+  else if (vecs <= 4) QUANT_GROUPS(4);
+  else if (vecs <= 8) QUANT_GROUPS(8);
+  else if (vecs <= 16) QUANT_GROUPS(16);
+  else QUANT_GROUPS(32);
+#undef QUANT_GROUPS
 }
 
 MSGL_API int msgl_quant_fp8(const void* x, void* out_q, void* out_scale, int rows, int hidden, int group,

@@ -92,7 +92,35 @@ def test_a_norm_does_not_depend_on_the_rows_around():
         assert torch.equal(K.rms_norm(x[a:b].contiguous(), w, 1e-6), whole[a:b])
 
 
-@pytest.mark.parametrize("rows,inter", [(1, 8), (3, 1024), (3, 1032), (2, 4096), (2049, 4104), (2049, 10240), (2049, 10248),
+@pytest.mark.parametrize("rows,hidden,runs", [(2047, 512, False), (2048, 512, True), (4095, 1024, False), (4096, 1016, True),
+                                              (4096, 1032, False), (4100, 264, True)])
+def test_many_short_rows_quantised_as_few(rows, hidden, runs):
+    """A row's maximum does not depend on who takes it: the rows of a large call are those of small ones (``runs``: the form that the
+    large one takes)."""
+    from minisglang_rdna4_b200.ops import cuda as K
+
+    x = _rand(rows, hidden)
+    q, s = K.per_token_quant_fp8(x)
+    for a in (0, 1000, rows - 9):
+        part = K.per_token_quant_fp8(x[a:a + 9].contiguous())
+        assert torch.equal(part[0].view(torch.uint8), q[a:a + 9].view(torch.uint8)) and torch.equal(part[1], s[a:a + 9])
+
+
+@pytest.mark.parametrize("hidden", [2560, 2568, 4096, 4104, 8192, 8200])
+@pytest.mark.parametrize("quant", [False, True])
+def test_norm_without_a_residual(hidden, quant):
+    from minisglang_rdna4_b200.ops import cuda as K
+
+    x, w = _rand(7, hidden), _rand(hidden, seed=2)
+    want = x.double() * torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-6) * w.double()
+    got = K._rms(x, None, w, 1e-6, False, quant)
+    if quant:
+        _same_rows8(got, want.to(torch.bfloat16))
+    else:   # one rounding to 16 bits of a product whose factors are good to fp32
+        assert float(((got.double() - want).abs() / want.abs().clamp_min(1e-6)).max()) <= 2.0 ** -8 * 1.01
+
+
+@pytest.mark.parametrize("rows,inter", [(1, 8), (2049, 1408), (2049, 2048), (2049, 2056), (3, 1024), (3, 1032), (2, 4096), (2049, 4104), (2049, 10240), (2049, 10248),
                                         (2, 12288), (2, 12296), (2, 20480), (2, 20488), (1, 28672)])
 def test_gated_activation_quantised(rows, inter):
     from minisglang_rdna4_b200.ops import cuda as K
