@@ -539,10 +539,12 @@ paged_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArg
   }
 }
 
-// Merges the parts of split attention: a CTA per query row, a warp per head, parts in ascending order and the loads of
+// Merges the parts of split attention: a warp per head of a query row, parts in ascending order and the loads of
 // several under way together. Splits: [split][row][head] in the workspace. DEALT: the slots of the workers that share a head; a
 // head of one worker is stored already. out_q (or null): the whole row once more, as e4m3 with one scale, which is
-// what a product with 8-bit rows takes: no kernel of its own then has to read the row again.
+// what a product with 8-bit rows takes: no kernel of its own then has to read the row again. With out_q a CTA has a whole row, for the
+// maximum; without, few rows are spread over the SMs, down to four heads a CTA (more CTAs than SMs, which start while the attention
+// kernel still runs, would take the room of its last ones: 96 requests 93 -> 116 us).
 template <typename T, int D, bool DEALT>
 __global__ void __launch_bounds__(D == 256 ? 512 : 1024) attn_combine_kernel(const AttnArgs args, uint8_t* __restrict__ out_q,
                                                                              float* __restrict__ out_scale) {
@@ -551,7 +553,7 @@ __global__ void __launch_bounds__(D == 256 ? 512 : 1024) attn_combine_kernel(con
   constexpr int AHEAD = D == 256 ? 3 : D == 128 ? 6 : 8;   // parts whose loads are under way together
   __shared__ float scratch[32];
   const int r = blockIdx.x, lane = threadIdx.x & 31, warps = blockDim.x >> 5, G = args.Hq / args.Hk;
-  if (r >= args.cu_q[args.B] && r < args.total_q) {
+  if (blockIdx.y == 0 && r >= args.cu_q[args.B] && r < args.total_q) {
     // a row of no request (padding of a captured batch): nobody wrote parts of it
     const size_t at = (size_t)r * args.Hq * D;
     for (int i = threadIdx.x * 8; i < args.Hq * D; i += blockDim.x * 8) {
@@ -563,7 +565,7 @@ __global__ void __launch_bounds__(D == 256 ? 512 : 1024) attn_combine_kernel(con
   if (DEALT ? r >= args.B : r >= args.cu_q[args.B]) return;
   const int q_row = DEALT ? args.cu_q[r] : r;
   float amax = 0.f;
-  for (int head = threadIdx.x >> 5; head < args.Hq; head += warps) {
+  for (int head = blockIdx.y * warps + (threadIdx.x >> 5); head < args.Hq; head += warps * gridDim.y) {
     const int2 who = DEALT ? args.shared[r * args.Hk + head / G] : make_int2(0, args.splits - 1);
     T* const dst = reinterpret_cast<T*>(args.out) + ((size_t)q_row * args.Hq + head) * D + lane * PER;
     float v[PER];
@@ -988,6 +990,17 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs a
   }
 }
 
+template <typename T, int D, bool DEALT>
+void launch_combine(const AttnArgs& a, int rows, void* out_q, void* out_scale, cudaStream_t stream) {
+  const int most = D == 256 ? 16 : 32;   // warps of a CTA
+  int warps = a.Hq < most ? a.Hq : most, ctas = 1;
+  if (out_q == nullptr) {
+    for (; warps > 4 && (long long)rows * ((a.Hq + warps / 2 - 1) / (warps / 2)) <= 148; warps /= 2)
+      ctas = (a.Hq + warps / 2 - 1) / (warps / 2);
+  }
+  msgl_launch(attn_combine_kernel<T, D, DEALT>, dim3(rows, ctas), dim3(warps * 32), 0, stream, a, (uint8_t*)out_q, (float*)out_scale);
+}
+
 // ------------------------------------------------------------------------------------------
 // Decode steps, dealt evenly. Every warp is a worker of its own: it keeps two stages of 32 KV tokens, issues the TMA copies of the
 // tile after next itself once it has used a stage up, and has an equal contiguous range of the (request, head, tile) units of the
@@ -1327,8 +1340,7 @@ int launch_deal(const CUtensorMap& map, const AttnArgs& a, void* out_q, void* ou
   if (most < (long long)ctas * kWorkers) ctas = (int)((most + kWorkers - 1) / kWorkers);
   if (ctas < 1) ctas = 1;
   msgl_launch(paged_decode_deal_kernel<T, KV8, D, EXT>, dim3(ctas), dim3(kWorkers * 32), smem, stream, map, a);
-  msgl_launch(attn_combine_kernel<T, D, true>, dim3(a.total_q > a.B ? a.total_q : a.B), dim3(a.Hq < 32 ? a.Hq * 32 : 1024), 0, stream,
-              a, (uint8_t*)out_q, (float*)out_scale);
+  launch_combine<T, D, true>(a, a.total_q > a.B ? a.total_q : a.B, out_q, out_scale, stream);
   MSGL_CHECK_LAUNCH("paged_decode_deal");
   return MSGL_OK;
 }
@@ -1536,10 +1548,7 @@ MSGL_API int msgl_paged_attention(const void* kv_map, const void* q, void* out, 
   else return MSGL_BAD_ARG;
   if (rc) return rc;
   if (splits > 1) {
-    const int most = head_dim == 256 ? 16 : 32;   // warps
-#define COMBINE(T, D)                                                                                                             \
-  msgl_launch(attn_combine_kernel<T, D, false>, dim3(total_q), dim3((hq < most ? hq : most) * 32), 0, stream, a, (uint8_t*)out_q, \
-              (float*)out_scale)
+#define COMBINE(T, D) launch_combine<T, D, false>(a, total_q, out_q, out_scale, stream)
     if (dtype == MSGL_BF16) {
       if (head_dim == 128) COMBINE(__nv_bfloat16, 128);
       else if (head_dim == 256) COMBINE(__nv_bfloat16, 256);

@@ -121,6 +121,24 @@ def test_rows_in_8_bits_are_the_quantised_rows(hq, hk, fp8, kw):
     assert torch.equal(got[0].view(torch.uint8), want[0].view(torch.uint8)) and torch.equal(got[1], want[1])
 
 
+@pytest.mark.parametrize("rows", [1, 2, 4, 5, 9, 18, 19, 37, 38, 148, 149])
+@pytest.mark.parametrize("hq,hk", [(32, 8), (40, 8), (6, 6), (3, 1)])
+@pytest.mark.parametrize("kw", [dict(deal=True), dict(deal=False, splits=3)])
+def test_heads_of_a_row_over_several_ctas(rows, hq, hk, kw):
+    """Few rows have their heads merged by several CTAs, many by one: the same sums."""
+    lens = [600 + 37 * i % 300 for i in range(rows)]
+    c = _case(lens, hq, hk, 128, False)
+    got = _run(c, False, **kw)
+    one = torch.ones(hk, device="cuda")
+    want = _want(c[0], c[1], c[2], c[4], 0.1, one, one)
+    assert float((got.double() - want).norm()) <= 2.0 ** -8 * 1.5 * float(want.norm())
+    wide = _run(c, False, quant=True, **kw)       # (a CTA has the row)
+    from minisglang_rdna4_b200.ops import cuda as K
+
+    q, s = K.per_token_quant_fp8(got.view(rows, -1))
+    assert torch.equal(wide[0].view(torch.uint8), q.view(torch.uint8)) and torch.equal(wide[1], s)
+
+
 def test_graph_and_two_streams():
     c = _case(LENGTHS["ragged"], 32, 8, 128, True)
     one = torch.ones(8, device="cuda")
