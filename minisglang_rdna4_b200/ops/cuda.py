@@ -367,7 +367,7 @@ def paged_attention(q, k_cache, v_cache, block_table, cu_q, seq_lens, scale, *, 
         workers = int(lib().msgl_paged_decode_workers(b, hq, hk, d, ps, int(fp8), int(ext), _dt(q)))
         if workers > 0:
             need = 2 * workers * (hq // hk) * (d + 1) + 2 * b * hk + 2
-            if workspace is None or workspace.numel() < need:
+            if workspace is None or workspace.numel() < need or workspace.data_ptr() % 16:
                 workspace = torch.empty(need, dtype=torch.float32, device=q.device)
             out = torch.empty_like(q)
             out_q, out_s = _row8(q) if quant else (None, None)
@@ -381,7 +381,7 @@ def paged_attention(q, k_cache, v_cache, block_table, cu_q, seq_lens, scale, *, 
         splits = choose_splits(b, hk, max_kv, decode or max_q == 1)
     if splits > 1:
         need = int(lib().msgl_attn_workspace_floats(t, hq, d, splits))
-        if workspace is None or workspace.numel() < need:
+        if workspace is None or workspace.numel() < need or workspace.data_ptr() % 16:
             workspace = torch.empty(need, dtype=torch.float32, device=q.device)
     out = torch.empty_like(q)
     out_q, out_s = _row8(q) if quant and splits > 1 else (None, None)

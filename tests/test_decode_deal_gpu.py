@@ -139,6 +139,16 @@ def test_heads_of_a_row_over_several_ctas(rows, hq, hk, kw):
     assert torch.equal(wide[0].view(torch.uint8), q.view(torch.uint8)) and torch.equal(wide[1], s)
 
 
+@pytest.mark.parametrize("kw", [dict(deal=True), dict(deal=False, splits=4)])
+def test_a_workspace_at_any_address(kw):
+    """The merge reads 16 bytes at a time: a workspace that begins elsewhere is not used."""
+    c = _case(LENGTHS["ragged"], 32, 8, 128, False)
+    want = _run(c, False, **kw)
+    ws = torch.full((1 << 23,), float("nan"), device="cuda")
+    assert torch.equal(_run(c, False, workspace=ws[1:], **kw), want) and bool(ws.isnan().all())
+    assert torch.equal(_run(c, False, workspace=ws, **kw), want) and not bool(ws.isnan().all())
+
+
 def test_graph_and_two_streams():
     c = _case(LENGTHS["ragged"], 32, 8, 128, True)
     one = torch.ones(8, device="cuda")
