@@ -46,10 +46,10 @@ class PagedAttentionBackend(BaseAttnBackend):
         self.layered = bool(heads)
         self.device = device
         # The number of KV splits of a decode step, and whether its tiles are dealt to the SMs instead, depend only on
-        # the batch size and the longest sequence the pool can hold; the deal itself depends on the lengths of the
-        # requests, which padding rows do not enter. So a captured graph and an eager step of one size reduce in the same
-        # order and agree bit for bit. ``single_split`` pins it to one split (speculative verification must reproduce
-        # decode).
+        # the batch size and the longest sequence the pool can hold; the deal itself depends on the lengths of all
+        # requests of the step, which padding rows do not enter. So a captured graph and an eager step of one size reduce in
+        # the same order and agree bit for bit, but a request's sums may be cut elsewhere beside longer or shorter ones.
+        # ``single_split`` pins it to one split (speculative verification must reproduce decode).
         self.max_seq_len = max_seq_len
         self.single_split = single_split
         self._workspace: Optional[torch.Tensor] = None
@@ -119,7 +119,7 @@ class PagedAttentionBackend(BaseAttnBackend):
                     splits = K.talk_splits(md.seq_lens.numel(), q.shape[1], k_cache.shape[1], q.shape[2], reach)
                 else:
                     splits = K.choose_splits(md.seq_lens.numel(), k_cache.shape[1], reach, True)
-                    deal = K.deal_pays(md.seq_lens.numel(), k_cache.shape[1], splits, False)
+                    deal = K.deal_pays(md.seq_lens.numel(), k_cache.shape[1], splits, False, reach)
         return ops.paged_attention(q, k_cache, v_cache, md.block_table, md.cu_q, md.seq_lens, scale, causal=True,
                                    max_q=md.max_q, max_kv=md.max_kv, decode=md.decode,
                                    workspace=md.workspace if talk is None else self._talk_workspace, splits=splits,
@@ -148,8 +148,9 @@ class PagedAttentionBackend(BaseAttnBackend):
             from ..ops.cuda import choose_splits, deal_pays
 
             b = md.seq_lens.numel()
-            splits = choose_splits(b, self.hk, self.max_seq_len or md.max_kv, True)
-            deal = deal_pays(b, self.hk, splits, fp8)
+            longest = self.max_seq_len or md.max_kv
+            splits = choose_splits(b, self.hk, longest, True)
+            deal = deal_pays(b, self.hk, splits, fp8, min(longest, window) if window > 0 else longest)
         mask = md.mask_swa if (window and md.mask_swa is not None) else md.mask
         return ops.paged_attention(
             q, pool.k_cache(layer), pool.v_cache(layer), block_table, md.cu_q, md.seq_lens, scale,

@@ -55,6 +55,7 @@ struct AttnArgs {
   long long ldg;
   int2* shared;      // dealt decode: [B * Hk] first and last worker of a (request, head) that several share, else -1
   int table_rows;    // requests that its tables in shared memory have room for
+  int deal_workers;  // workers of the GPU
 };
 
 __device__ int g_attn_status = 0;
@@ -1012,12 +1013,17 @@ void launch_combine(const AttnArgs& a, int rows, void* out_q, void* out_scale, c
 // the end. Here all 12 (6) warps consume and finish together. B200, us, with the merge, splits -> dealt: 37 requests of 90 to 3500
 // tokens (fp8) 63.8 -> 49.7, 256 of 512 to 2304 182.5 -> 164.5, 4 of 20000 to 31000 (bf16) 115.3 -> 102.4. Summing the parts by
 // the worker that arrives last took 8 us more: one warp waits for a dozen parts while the rest of the GPU is idle.
+// Where no (request, head) is long against an equal share, none is shared: writing and summing the parts takes as long as some nine tiles
+// (six of 16-bit rows). fp8, 32 query and 8 key heads, splits at the time -> all shared -> this: 96 x 64 tokens 9.9 -> 12.4 -> 9.6,
+// 192 x 64 16.0 -> 20.8 -> 14.1, 192 x 300 35.9 -> 36.0 -> 30.4, 32 x 300 15.8 -> 17.4 -> 15.0, 256 x 300 42.7 -> 43.3 -> 43.3.
 // The deal depends on the lengths of the requests of at least two tiles alone; shorter ones, the padding rows of a captured
-// batch among them, are whole segments and are handed out round robin, so that padding changes nobody's bits.
+// batch among them, are whole segments and are handed out round robin, so that padding changes nobody's bits. The parts of a shared
+// request, and with them the order of its sum, depend on the lengths of the others.
 // ------------------------------------------------------------------------------------------
 constexpr int DTK = 32;           // KV tokens of a tile
 constexpr int kMostParts = 16;    // parts of a (request, head), about: two rounds of loads of attn_combine_kernel
 constexpr int kDealRows = 1024;   // requests of a call
+template <bool KV8> constexpr int kSumTiles = KV8 ? 9 : 6;   // tiles that a warp works off in the time that the sum of parts takes
 
 template <bool EXT> __device__ __forceinline__ int decode_tiles(const AttnArgs& a, int kv_len) {
   if (kv_len <= 0) return 0;
@@ -1097,8 +1103,8 @@ paged_decode_deal_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnA
   const uint32_t bars = smem_u32(smem) + kWorkers * 2 * STAGE_BYTES + warp * 16;
   uint8_t* const after = smem + kWorkers * (2 * STAGE_BYTES + 16);
   volatile int* const abort_flag = reinterpret_cast<volatile int*>(after) + warp;
-  int* const s_part = reinterpret_cast<int*>(after) + kWorkers;   // [2 * kWorkers]: sums and maxima of the warps
-  int* const len = s_part + 2 * kWorkers;
+  int* const s_part = reinterpret_cast<int*>(after) + kWorkers;   // [3 * kWorkers]: sums, maxima and numbers of the warps
+  int* const len = s_part + 3 * kWorkers;
   int* const row = len + args.table_rows;
   int* const pre = row + args.table_rows;
   const int G = args.Hq / args.Hk;
@@ -1116,7 +1122,7 @@ paged_decode_deal_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnA
     // lengths, and the tiles before each request: a run of requests per thread, a scan over the threads
     const int run = (args.B + kWorkers * 32 - 1) / (kWorkers * 32);
     const int b0 = min((int)threadIdx.x * run, args.B), b1 = min(b0 + run, args.B);
-    int mine = 0;
+    int mine = 0, count = 0;
 #pragma unroll 4
     for (int b = b0; b < b1; ++b) {
       const int l = args.seq_lens[b];
@@ -1124,6 +1130,7 @@ paged_decode_deal_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnA
       len[b] = l;
       const int t = decode_tiles<EXT>(args, l);
       mine += t > 1 ? t : 0;
+      count += t > 1;
       longest = max(longest, t);
     }
     int sum = mine;
@@ -1132,19 +1139,27 @@ paged_decode_deal_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnA
       const int up = __shfl_up_sync(0xffffffffu, sum, o);
       if (lane >= o) sum += up;
       longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
+      count += __shfl_xor_sync(0xffffffffu, count, o);
     }
-    if (lane == 31) { s_part[warp] = sum; s_part[kWorkers + warp] = longest; }
+    if (lane == 31) { s_part[warp] = sum; s_part[kWorkers + warp] = longest; s_part[2 * kWorkers + warp] = count; }
     __syncthreads();
-    int before = sum - mine;
+    int before = sum - mine, total = 0;
+    count = 0;
 #pragma unroll
     for (int w = 0; w < kWorkers; ++w) {
       if (w < warp) before += s_part[w];
+      total += s_part[w];
       longest = max(longest, s_part[kWorkers + w]);
+      count += s_part[2 * kWorkers + w];
     }
+    // a warp's tiles where every (request, head) stays whole, at most, against an equal share and what the sum of parts costs
+    const int whole = (count * args.Hk + args.deal_workers - 1) / args.deal_workers * longest;
+    const bool share = whole > total * args.Hk / args.deal_workers + kSumTiles<KV8>;
+    if (!share) before = 0;
     for (int b = b0; b < b1; ++b) {
       pre[b] = before;
       const int t = decode_tiles<EXT>(args, len[b]);
-      before += t > 1 ? t : 0;
+      before += share && t > 1 ? t : 0;
     }
     if (threadIdx.x == kWorkers * 32 - 1) pre[args.B] = before;
     __syncthreads();
@@ -1311,7 +1326,7 @@ int deal_rows(int B) { return B <= 256 ? 256 : B <= 512 ? 512 : kDealRows; }
 template <typename T, bool KV8, int D, bool EXT = false>
 int deal_ctas(int rows, int* smem) {
   constexpr int kWorkers = kWorkersOf<KV8, D>;
-  constexpr int fixed = kWorkers * (2 * 2 * (D * (KV8 ? 1 : 2) / 128) * DTK * 128 + 16) + 3 * kWorkers * 4 + 1024;
+  constexpr int fixed = kWorkers * (2 * 2 * (D * (KV8 ? 1 : 2) / 128) * DTK * 128 + 16) + 4 * kWorkers * 4 + 1024;
   *smem = fixed + (3 * rows + 1) * 4;
   static int ctas[3] = {0, 0, 0};   // of 256, 512, 1024 table rows
   const int at = rows == 256 ? 0 : rows == 512 ? 1 : 2;
@@ -1330,11 +1345,12 @@ int deal_ctas(int rows, int* smem) {
 }
 
 template <typename T, bool KV8, int D, bool EXT = false>
-int launch_deal(const CUtensorMap& map, const AttnArgs& a, void* out_q, void* out_scale, cudaStream_t stream) {
+int launch_deal(const CUtensorMap& map, AttnArgs a, void* out_q, void* out_scale, cudaStream_t stream) {
   constexpr int kWorkers = kWorkersOf<KV8, D>;
   int smem = 0;
   int ctas = deal_ctas<T, KV8, D, EXT>(a.table_rows, &smem);
   if (ctas < 0) return MSGL_CUDA_ERROR;
+  a.deal_workers = ctas * kWorkers;
   // never more warps than there can be tiles (which leaves the deal as it is)
   const long long most = (long long)a.B * a.Hk * (((long long)a.bt_stride * a.page_size + DTK - 1) / DTK);
   if (most < (long long)ctas * kWorkers) ctas = (int)((most + kWorkers - 1) / kWorkers);
@@ -1540,6 +1556,7 @@ MSGL_API int msgl_paged_attention(const void* kv_map, const void* q, void* out, 
   a.status = status;
   a.shared = nullptr;
   a.table_rows = 0;
+  a.deal_workers = 0;
   const CUtensorMap& map = *reinterpret_cast<const CUtensorMap*>(kv_map);
   int rc;
   if (ext) rc = dispatch_attn_ext<__nv_bfloat16>(map, a, head_dim, max_q, stream);

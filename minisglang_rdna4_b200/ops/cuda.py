@@ -306,14 +306,21 @@ def _row8(q):
             torch.empty((t,), dtype=torch.float32, device=q.device))
 
 
-def deal_pays(batch, hk, splits, fp8):
+def deal_pays(batch, hk, splits, fp8, longest):
     """Whether a decode step's tiles are better dealt out by the lengths (``paged_decode_deal_kernel``) than cut into ``splits``
-    for each request. B200, us, cut -> dealt: few requests have few tiles, and the deal's tables cost more than it evens
-    out (fp8, 8 key heads: 1 x 700 tokens 15.1 -> 19.2, 8 x 300 15.9 -> 18.9, 16 x 4000 45.7 -> 48.3); with 32 equal ones it
-    costs 5 (51.3 -> 56.7), with unequal ones it gains three times that (37 x 90 to 3500 63.8 -> 49.7, 256 x 512 to 2304
-    182.5 -> 164.5). Few long ones: where the splits need a second wave (4 x 20000 to 31000 bf16, 512 CTAs of which 444 fit,
-    115.3 -> 102.4)."""
-    return batch * hk >= 192 or batch * hk * splits > (888 if fp8 else 444)
+    for each request; ``longest``: the most tokens that a request of the pool can have. It follows nothing of the step but the batch size, so
+    that a captured step and an eager one agree.
+
+    B200, us with the merge and, for fp8, the rows in 8 bits, cut -> dealt; longest request first, which is the scheduler's order, and
+    (equal lengths) of the same mean. fp8, 32 query and 8 key heads, 512 to 2304 tokens: 16 requests 23.7 -> 23.5 (20.7 -> 22.9),
+    24 29.7 -> 25.4 (24.2 -> 25.8), 32 38.2 -> 28.9 (29.9 -> 27.9), 64 53.1 -> 41.7 (47.4 -> 41.6), 128 82.1 -> 71.6 (81.6 -> 71.6), 256
+    138.6 -> 136.3 (132.9 -> 134.4); shuffled, 256: 172 -> 136. So from 24 requests of 8 heads on. 16 bits: half the warps fit, and the cut
+    has all heads of one request side by side: it wins where one split is enough (96 83.8 -> 93.9, 128 116.5 -> 124.3), with more it is
+    even (32 39.6 -> 38.6, 64 67.5 -> 65.3 (72.3 -> 64.9), 48 49.5 -> 51.4). Few requests: the cut, whose tables cost less (4 x 512 to 2304
+    11.2 -> 15.6), unless they can be long and the splits need a second wave (4 x 20000 to 31000, 512 CTAs of which 444 fit, 94.5 -> 78.8)."""
+    if longest >= 16384 and batch * hk * splits > (888 if fp8 else 444):
+        return fp8 or splits > 1
+    return batch * hk >= 192 and (fp8 or splits > 1)
 
 
 def choose_splits(batch, hk, max_kv, decode):

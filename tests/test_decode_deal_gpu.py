@@ -58,6 +58,9 @@ LENGTHS = {
     "one_tile": [1], "no_tiles": [0, 5, 0], "edge": [64, 65, 128, 129, 1], "alone": [700], "long": [40000],
     "ragged": [90, 3500, 64, 1, 1200, 65, 2500, 0, 333], "many": [(37 * i) % 500 + 1 for i in range(300)],
     "shortest": [64] * 40, "two": [20000, 70],
+    # no request shared: more of them than warps, and fewer; the longest one just long enough to be shared, and a tile less
+    "whole": [300 - i % 40 for i in range(96)], "whole_few": [200, 1, 64, 0, 150] * 8,
+    "slack": [320, *[64] * 30], "slack_less": [288, *[64] * 30], "slack16": [224, *[64] * 30], "slack16_less": [192, *[64] * 30],
 }
 
 
@@ -78,8 +81,9 @@ def test_against_64_bits(name, hq, hk, d, fp8):
     assert K.attn_status() == 0
 
 
-def test_padding_rows_change_nothing():
-    lens = LENGTHS["ragged"]
+@pytest.mark.parametrize("name", ["ragged", "whole", "whole_few", "slack", "slack_less"])
+def test_padding_rows_change_nothing(name):
+    lens = LENGTHS[name]
     q, pool, table, cu, n = _case(lens, 32, 8, 128, True)
     one = torch.ones(8, device="cuda")
     alone = _run((q, pool, table, cu, n), True, scales=(one, one))
