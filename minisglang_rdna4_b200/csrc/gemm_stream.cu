@@ -20,7 +20,7 @@
 //   2560 x 9728 mxfp4       2.0     27.9 -> 12.3 (7.8)      27.8 -> 13.6 (8.1)      28.0 -> 20.5 (9.2)
 //   6144 x 2560 mxfp4       1.3     13.0 -> 9.6             12.2 -> 10.0            10.4 -> 14.5
 // Where the bytes are few, what is left is the summing of shared tiles (a store, a ticket and a load through L2, about
-// 4 us and 0.05 us a row); the 64-row 4-bit products stay with the tiled kernel (ops/cuda.py, _stream_pays).
+// 4 us and 0.05 us a row): up to how many rows a product is taken follows its tiles and K blocks (ops/cuda.py, _stream_rows).
 #include "common.cuh"
 #include "ptx.cuh"
 

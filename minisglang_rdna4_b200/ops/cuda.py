@@ -791,15 +791,45 @@ def _stream_counters(device, tiles: int) -> torch.Tensor:
         return got
 
 
-def _stream_pays(m: int, weight_bytes: int, planes: bool) -> bool:
-    """Whether ``csrc/gemm_stream.cu`` is the faster one. Unreduced sums: up to 128 rows (B200, K = 12288 of 4096 16-bit
-    columns: 21.7 against 31 us at 64 rows; at 256 its eight planes cost the next norm what the product gains). Finished
-    sums: tiles that CTAs share are summed by one of them, about 4 us and 0.05 us a row, which up to 32 rows the even deal
-    always makes up for (6144 x 2560 in 4 bits: 10.0 against 12.2 us at 16 rows, 14.5 against 10.4 at 64), up to 64 rows
-    where there are enough bytes to deal (24576 x 4096 in 16 bits: 42.7 against 48.7 us at 64 rows, 52 against 51 at 128)."""
-    if planes:
-        return m <= 128
-    return m <= 32 or (m <= 64 and weight_bytes >= 48 << 20)
+# us on B200, by kind of weights, with tiles of 128 weight rows, K blocks of 128 bytes and p CTAs that share a tile:
+# csrc/gemm_tcgen05.cu t0 + blocks (a waves + b tiles / SMs), csrc/gemm_stream.cu c0 + c1 rows + p (c2 + c3 rows) + d blocks tiles.
+# Fitted to both kernels' finished sums: 128 to 151936 columns, K of 512 to 28672, 1 to 64 rows, weights not in L2.
+_SMS = 148
+_STREAM_COST = {KIND_F16: (3.6, 0.243, 0.18, 5.4, 0.046, 0.19, 0.010, 0.0025),
+                KIND_BF16: (3.6, 0.243, 0.18, 5.4, 0.046, 0.19, 0.010, 0.0025),
+                KIND_F8: (3.6, 0.23, 0.25, 4.5, 0.034, 0.25, 0.0115, 0.00275),
+                KIND_MXF4: (3.3, 0.288, 0.144, 4.3, 0.035, 0.24, 0.0115, 0.0029)}
+_STREAM_ROWS: Dict[Tuple[int, int, int, bool], int] = {}
+
+
+def _stream_rows(kind: int, n: int, k: int, planes: bool) -> int:
+    """Rows up to which ``csrc/gemm_stream.cu`` is the faster one for a weight matrix.
+
+    Finished sums: an even deal of the bytes, and a sum of the shared tiles, against a chain through all of K in whole tiles. It gains most where
+    tiles fill few SMs and K is long (8 bits, 16 rows, 4096 x 12288 30 -> 16 us) and loses where they fill them (16384 x 8192 28 -> 30)
+    or K is short (1000 x 1216 5.5 -> 8; below 2048 only more tiles than SMs make up for it). Above 32 rows matrices of 48 MB and more
+    (24576 x 4096 in 16 bits, 64 rows, 48.8 -> 42.4), none above 64 (52 against 51 at 128). Over the shapes of the fit the choice is 1 % from the better one up
+    to 32 rows on average, and 32 rows for every shape 1 to 12 %.
+
+    Unreduced sums: up to 128 rows (at 256 the eight planes cost the next norm what the product gains), from K = 2048 on; for shorter
+    ones the ranges of the split-K plan do as well or better (8 bits, 128 rows, 1000 x 1216 7.5 -> 9.6 us with the norm)."""
+    key = (kind, n, k, planes)
+    rows = _STREAM_ROWS.get(key)
+    if rows is None:
+        tiles, wide = -(-n // 128), kind in (KIND_F16, KIND_BF16)
+        if planes:
+            rows = 128 if k >= 2048 else 0
+        elif k < 2048 and tiles <= _SMS:
+            rows = 0
+        else:
+            t0, a, b, c0, c1, c2, c3, d = _STREAM_COST[kind]
+            blocks = -(-k // (64 if wide else 128))
+            shared = max(1.0, min(_SMS, tiles * blocks // 4) / tiles)
+            gain = t0 + blocks * (a * -(-tiles // _SMS) + b * tiles / _SMS) - c0 - c2 * shared - d * blocks * tiles
+            large = n * k * (4 if wide else 2 if kind == KIND_F8 else 1) >= 96 << 20
+            rows = max(0, min(64 if large else 32, int(gain / (c1 + c3 * shared))))
+        _STREAM_ROWS[key] = rows
+    return rows
 
 
 def _decode_step() -> bool:
@@ -847,7 +877,7 @@ def _gemm(kind, a, b, n, k, out_dtype, a_scale=None, b_scale=None, bias=None, sf
     global _PENDING_PLANES
     want_planes, _PENDING_PLANES = _PENDING_PLANES, False
     want_planes = want_planes and n <= PLANES_MOST_COLUMNS
-    if (0 < m <= 128 and bn == 0 and not max_ctas and not SPLIT_K and _stream_pays(m, b.nbytes, want_planes)
+    if (0 < m <= 128 and bn == 0 and not max_ctas and not SPLIT_K and m <= _stream_rows(kind, n, k, want_planes)
             and (few or _decode_step())):
         return _gemm_stream(kind, a, b, m, n, k, out_dtype, a_scale, b_scale, bias, sf_atoms, want_planes)
     if want_planes and 0 < m <= 256 and bn == 0:

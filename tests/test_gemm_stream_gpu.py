@@ -173,6 +173,27 @@ def test_counters_of_many_streams_and_captures(monkeypatch):
     assert K._stream_counters("cuda", 8) is not small and len(K._CAPTURE_COUNTERS[("cuda", 5)][1]) == 1
 
 
+def test_which_products_it_takes(monkeypatch):
+    from minisglang_rdna4_b200.ops import cuda as K
+
+    for kind in range(4):
+        for n in (8, 128, 1000, 2560, 12288, 18944, 18952, 151936):
+            for k in (128, 1216, 2048, 4096, 28672):
+                rows = K._stream_rows(kind, n, k, False)
+                assert 0 <= rows <= (64 if n * k * (2, 2, 1, 0.5)[kind] >= 48 << 20 else 32)
+                assert rows == 0 or k >= 2048 or n > 148 * 128
+                assert K._stream_rows(kind, n, k, True) == (128 if k >= 2048 else 0)
+    # few tiles and a long chain; as many tiles as SMs; a short chain
+    assert K._stream_rows(1, 2560, 9728, False) == 32 and K._stream_rows(1, 4096, 12288, False) == 64
+    assert K._stream_rows(3, 16384, 4096, False) < 16 and K._stream_rows(2, 1000, 1216, False) == 0
+    taken = []
+    monkeypatch.setattr(K, "_gemm_stream", lambda kind, a, b, m, *r: taken.append(m) or torch.empty(m, b.shape[0], device="cuda"))
+    w = torch.zeros(2560, 9728, device="cuda", dtype=torch.bfloat16)
+    for m in (0, 1, 32, 33):
+        K.gemm(torch.zeros(m, 9728, device="cuda", dtype=torch.bfloat16), w, None, torch.float32, few=True)
+    assert taken == [1, 32]
+
+
 def test_operands_it_does_not_take_are_refused():
     from minisglang_rdna4_b200.ops import cuda as K
     from minisglang_rdna4_b200.ops._lib import lib
