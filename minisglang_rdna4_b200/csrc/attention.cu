@@ -543,9 +543,9 @@ paged_attention_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArg
 // Merges the parts of split attention: a warp per head of a query row, parts in ascending order and the loads of
 // several under way together. Splits: [split][row][head] in the workspace. DEALT: the slots of the workers that share a head; a
 // head of one worker is stored already. out_q (or null): the whole row once more, as e4m3 with one scale, which is
-// what a product with 8-bit rows takes: no kernel of its own then has to read the row again. With out_q a CTA has a whole row, for the
-// maximum; without, few rows are spread over the SMs, down to four heads a CTA (more CTAs than SMs, which start while the attention
-// kernel still runs, would take the room of its last ones: 96 requests 93 -> 116 us).
+// what a product with 8-bit rows takes: no kernel of its own then has to read the row again. With out_q a CTA has a whole row,
+// for the maximum; without, few rows are spread over the SMs, down to four heads a CTA (more CTAs than SMs, which start while the
+// attention kernel still runs, would take the room of its last ones: 96 requests 93 -> 116 us).
 template <typename T, int D, bool DEALT>
 __global__ void __launch_bounds__(D == 256 ? 512 : 1024) attn_combine_kernel(const AttnArgs args, uint8_t* __restrict__ out_q,
                                                                              float* __restrict__ out_scale) {
@@ -1013,8 +1013,8 @@ void launch_combine(const AttnArgs& a, int rows, void* out_q, void* out_scale, c
 // the end. Here all 12 (6) warps consume and finish together. B200, us, with the merge, splits -> dealt: 37 requests of 90 to 3500
 // tokens (fp8) 63.8 -> 49.7, 256 of 512 to 2304 182.5 -> 164.5, 4 of 20000 to 31000 (bf16) 115.3 -> 102.4. Summing the parts by
 // the worker that arrives last took 8 us more: one warp waits for a dozen parts while the rest of the GPU is idle.
-// Where no (request, head) is long against an equal share, none is shared: writing and summing the parts takes as long as some nine tiles
-// (six of 16-bit rows). fp8, 32 query and 8 key heads, splits at the time -> all shared -> this: 96 x 64 tokens 9.9 -> 12.4 -> 9.6,
+// Where no (request, head) is long against an equal share, none is shared: writing and summing the parts takes as long as some
+// nine tiles (six of 16-bit rows). fp8, 32 query and 8 key heads, us, splits -> all shared -> this: 96 x 64 tokens 9.9 -> 12.4 -> 9.6,
 // 192 x 64 16.0 -> 20.8 -> 14.1, 192 x 300 35.9 -> 36.0 -> 30.4, 32 x 300 15.8 -> 17.4 -> 15.0, 256 x 300 42.7 -> 43.3 -> 43.3.
 // The deal depends on the lengths of the requests of at least two tiles alone; shorter ones, the padding rows of a captured
 // batch among them, are whole segments and are handed out round robin, so that padding changes nobody's bits. The parts of a shared

@@ -72,8 +72,9 @@ MSGL_API int msgl_embedding(const void* ids, const void* w, void* out, int rows,
 // would follow): two vectors a thread, so that a decode step's few rows have all their bytes under way too, four above 4096 columns,
 // where 512 and more threads a row leave too few rows on an SM, and without a residual, which halves the bytes of a row, above 2560.
 // B200, us, with the residual and e4m3 out, before -> after: 1 x 2560 3.9 -> 2.7, 64 x 4096 4.7 -> 3.1, 8190 x 2560 31.5 -> 30.3,
-// 8190 x 8192 120 -> 107, 8190 x 12288 255 -> 200, 16 bits out 256 -> 140; without a residual 8190 x 8192 76 -> 64 (two vectors: 82), 8190 x 12288
-// 117 -> 98 (157), 8190 x 4096 32.0 -> 32.7 (35.1), 16 x 4096 2.8 -> 2.0; 5 planes of 64 x 4096 7.6 -> 4.5, 3 of 32 x 8192 11.9 -> 4.9.
+// 8190 x 8192 120 -> 107, 8190 x 12288 255 -> 200, 16 bits out 256 -> 140; without a residual 8190 x 8192 76 -> 64 (two
+// vectors: 82), 8190 x 12288 117 -> 98 (157), 8190 x 4096 32.0 -> 32.7 (35.1), 16 x 4096 2.8 -> 2.0; 5 planes of 64 x 4096
+// 7.6 -> 4.5, 3 of 32 x 8192 11.9 -> 4.9.
 // ------------------------------------------------------------------------------------------
 template <typename T, bool ADD, bool QUANT, int VPT, int MAXT, bool PLANES = false>
 __global__ void __launch_bounds__(MAXT) rms_norm_kernel(const T* __restrict__ x, T* __restrict__ residual,
@@ -426,9 +427,9 @@ MSGL_API int msgl_act_and_mul(const void* x, void* out, void* out_q, void* out_s
 // stand-alone activation quantisers: per token (group == hidden) or per `group` elements
 // ------------------------------------------------------------------------------------------
 // A group is one row of up to 16384 elements (a CTA each, VPT 16-byte vectors a thread, read once), or a run of
-// elements of any multiple of 8 (a power of two of lanes each, vectors 16 bytes a lane). Many short rows are runs too: a CTA of one or
-// two warps for each costs more than it reads (8190 x 512 4.2 us against 8.9, 8190 x 1024 6.6 against 9.0; 2397 x 1024 3.5 against 2.9). B200, us, a warp for each group of any
-// length and two passes over it -> now: 1 x 4096 3.7 -> 1.8, 256 x 4096 5.1 -> 2.7, 8192 x 8192 53 -> 38; 16640 x 2048 in groups of 128
+// elements of any multiple of 8 (a power of two of lanes each, vectors 16 bytes a lane). Many short rows are runs too: a CTA of
+// one or two warps for each costs more than it reads (8190 x 512 8.9 us, as runs 4.2; 8190 x 1024 9.0, 6.6; but 2397 x 1024 2.9, 3.5).
+// B200, us, a warp for each group of any length and two passes over it -> now: 1 x 4096 3.7 -> 1.8, 256 x 4096 5.1 -> 2.7, 8192 x 8192 53 -> 38; 16640 x 2048 in groups of 128
 // 51 -> 33.
 template <typename T, int VPT>
 __global__ void __launch_bounds__(512) quant_row_kernel(const T* __restrict__ x, uint8_t* __restrict__ out_q,

@@ -23,11 +23,12 @@
 // Bound of many rows: what an SM takes in from L2, 32 KB for each K block of a tile (with the MMAs, the promotion and the stores all
 // left out a block still takes 0.49 us, 65 GB/s an SM). On top of that came the stores: a lane wrote 16 bytes of its own row at a time,
 // a quarter of the time of the first product and 30 % of the second. A warp now packs its 32 x 64 results into shared memory and
-// leaves them to one TMA store, whose end it waits for before the next tile's. Eight promotion warps of 64 columns each were 2 to 4 %
-// slower than four (4096 x 4096, 100 rows 17.1 -> 16.5 us; 24576 x 4096, 1024 rows 159 -> 154), two partial buffers with a sixth stage up to 5 %
-// slower than four with five for many rows.
-// B200, us, stores of the lanes -> this: 24576 x 4096, 4096 rows 647 -> 593, 1024 rows 173 -> 154, 100 rows 33.6 -> 31.9; 1536 x 2048, 4096
-// rows 29.2 -> 25.1; 4096 x 4096, 128 rows 16.5 -> 16.6, 16 rows 15.4 -> 16.1 (a store's end is waited for).
+// leaves them to one TMA store, whose end it waits for before the next tile's. Eight promotion warps of 64 columns each were 2
+// to 4 % slower than four (4096 x 4096, 100 rows 17.1 us, 16.5 with four; 24576 x 4096, 1024 rows 159, 154), two partial buffers
+// and six stages up to 5 % slower than four and five for many rows.
+// B200, us, stores of the lanes -> this, weights not in L2: 24576 x 4096, 4096 rows 650 -> 576, 1024 rows 178 -> 158, 100 rows
+// 36.5 -> 34.5; 1536 x 2048, 4096 rows 29.5 -> 25.6, 128 rows 11.2 -> 10.1; 4096 x 4096, 4096 rows 111 -> 100, 128 rows 17.1 -> 17.0. Up to 16
+// rows it costs 3 % (1536 x 2048 9.3 -> 9.7, 4096 x 4096 16.0 -> 16.5): the end of a store is waited for.
 #include "common.cuh"
 #include "ptx.cuh"
 

@@ -220,9 +220,9 @@ struct ArgMaxPlan {
 // A share of less than 2048 values is one round of loads: nothing to split. Clusters of CTAs that do not all fit at once start in
 // rounds, so a row has as many CTAs as keep the whole within the SMs; of wide rows up to four CTAs of 512 threads on an SM, whose loads
 // make up for that. Up to two rows for each SM, one CTA a row of the form that fits twice.
-// B200, us, 1024 threads a row -> this: 151936 columns, 1 row 13.7 -> 3.6, 16 14.2 -> 4.9, 48 14.3 -> 6.7, 64 14.4 -> 7.8 (clusters of 8: 10.5), 100
-// 14.4 -> 9.9, 150 24.1 -> 19.6, 256 28.9 -> 27.2 (without the form for two: 34); 16384 columns, 1 row 2.6 -> 2.2, 64 2.9 -> 2.8 (clusters of 8: 5.4),
-// 256 4.2 -> 4.1; 32000, 64 4.3 -> 3.5, 256 6.1 -> 6.2.
+// B200, us, 1024 threads a row -> this: 151936 columns, 1 row 13.7 -> 3.6, 16 14.2 -> 4.9, 37 14.3 -> 6.4, 64 14.4 -> 7.9 (clusters
+// of 8: 10.5), 100 14.4 -> 9.6, 150 24.1 -> 19.0, 256 28.9 -> 27.2 (without the form for two: 34); 16384 columns, 1 row 2.6 -> 2.2,
+// 64 2.9 -> 2.8 (clusters of 8: 5.4), 256 4.2 -> 4.1; 32000, 64 4.3 -> 3.5, 256 6.1 -> 6.2.
 ArgMaxPlan argmax_plan(int rows, int vocab) {
   constexpr int sms = 148;
   const bool two = rows > sms && rows <= 2 * sms;

@@ -308,16 +308,17 @@ def _row8(q):
 
 def deal_pays(batch, hk, splits, fp8, longest):
     """Whether a decode step's tiles are better dealt out by the lengths (``paged_decode_deal_kernel``) than cut into ``splits``
-    for each request; ``longest``: the most tokens that a request of the pool can have. It follows nothing of the step but the batch size, so
-    that a captured step and an eager one agree.
+    for each request; ``longest``: the most tokens that a request of the pool can have. It follows nothing of the step but
+    the batch size, so that a captured step and an eager one agree.
 
-    B200, us with the merge and, for fp8, the rows in 8 bits, cut -> dealt; longest request first, which is the scheduler's order, and
-    (equal lengths) of the same mean. fp8, 32 query and 8 key heads, 512 to 2304 tokens: 16 requests 23.7 -> 23.5 (20.7 -> 22.9),
-    24 29.7 -> 25.4 (24.2 -> 25.8), 32 38.2 -> 28.9 (29.9 -> 27.9), 64 53.1 -> 41.7 (47.4 -> 41.6), 128 82.1 -> 71.6 (81.6 -> 71.6), 256
-    138.6 -> 136.3 (132.9 -> 134.4); shuffled, 256: 172 -> 136. So from 24 requests of 8 heads on. 16 bits: half the warps fit, and the cut
-    has all heads of one request side by side: it wins where one split is enough (96 83.8 -> 93.9, 128 116.5 -> 124.3), with more it is
-    even (32 39.6 -> 38.6, 64 67.5 -> 65.3 (72.3 -> 64.9), 48 49.5 -> 51.4). Few requests: the cut, whose tables cost less (4 x 512 to 2304
-    11.2 -> 15.6), unless they can be long and the splits need a second wave (4 x 20000 to 31000, 512 CTAs of which 444 fit, 94.5 -> 78.8)."""
+    B200, us with the merge and, for fp8, the rows in 8 bits, cut -> dealt; longest request first, which is the scheduler's
+    order, and (equal lengths) of the same mean. fp8, 32 query and 8 key heads, 512 to 2304 tokens: 16 requests 23.7 -> 23.5
+    (20.7 -> 22.9), 24 29.7 -> 25.4 (24.2 -> 25.8), 32 38.2 -> 28.9 (29.9 -> 27.9), 64 53.1 -> 41.7 (47.4 -> 41.6), 128 82.1 -> 71.6
+    (81.6 -> 71.6), 256 138.6 -> 136.3 (132.9 -> 134.4); shuffled, 256: 172 -> 136. So from 24 requests of 8 heads on. 16 bits: half
+    the warps fit, and the cut wins where one split is enough (96 83.8 -> 93.9, 128 116.5 -> 124.3), with more it is even (32
+    39.6 -> 38.6, 64 67.5 -> 65.3 (72.3 -> 64.9), 48 49.5 -> 51.4). Few requests: the cut, whose tables cost less (4 x 512 to 2304
+    11.2 -> 15.6), unless they can be long and the splits need a second wave (4 x 20000 to 31000, 512 CTAs of which 444 fit,
+    94.5 -> 78.8)."""
     if longest >= 16384 and batch * hk * splits > (888 if fp8 else 444):
         return fp8 or splits > 1
     return batch * hk >= 192 and (fp8 or splits > 1)
@@ -769,7 +770,8 @@ def _stream_counters(device, tiles: int) -> torch.Tensor:
 
     A capture has sets of its own, zeroed by the graph in front of the first product that uses them: memory of a graph's
     pool belongs to the other graphs of the pool too, graphs are replayed in any order and on any stream, and a fill that
-    is captured is not run. They are kept until the stream is in another capture: until then they must not be reused, after that they may."""
+    is captured is not run. They are kept until the stream is in another capture: for the rest of their own one nothing else
+    may have their memory, and afterwards every replay fills them again."""
     stream = _stream()
     key, capture, numel = (device, stream), _capture_id(stream), max(2 * tiles, 4096)
     with _STREAM_COUNTERS_LOCK:
@@ -805,11 +807,12 @@ _STREAM_ROWS: Dict[Tuple[int, int, int, bool], int] = {}
 def _stream_rows(kind: int, n: int, k: int, planes: bool) -> int:
     """Rows up to which ``csrc/gemm_stream.cu`` is the faster one for a weight matrix.
 
-    Finished sums: an even deal of the bytes, and a sum of the shared tiles, against a chain through all of K in whole tiles. It gains most where
-    tiles fill few SMs and K is long (8 bits, 16 rows, 4096 x 12288 30 -> 16 us) and loses where they fill them (16384 x 8192 28 -> 30)
-    or K is short (1000 x 1216 5.5 -> 8; below 2048 only more tiles than SMs make up for it). Above 32 rows matrices of 48 MB and more
-    (24576 x 4096 in 16 bits, 64 rows, 48.8 -> 42.4), none above 64 (52 against 51 at 128). Over the shapes of the fit the choice is 1 % from the better one up
-    to 32 rows on average, and 32 rows for every shape 1 to 12 %.
+    Finished sums: an even deal of the bytes, and a sum of the shared tiles, against a chain through all of K in whole tiles.
+    It gains most where tiles fill few SMs and K is long (8 bits, 16 rows, 4096 x 12288 30 -> 16 us) and loses where they fill
+    them (16384 x 8192 28 -> 30) or K is short (1000 x 1216 5.5 -> 8; below 2048 only more tiles than SMs make up for it). Above
+    32 rows matrices of 48 MB and more (24576 x 4096 in 16 bits, 64 rows, 48.8 -> 42.4), none above 64 (128: 51 -> 52). Over the
+    shapes of the fit the choice is 1 % from the better one up to 32 rows on average, and 32 rows for every shape 1 to 12 %; the worst
+    is 12288 x 4096 (96 tiles) at 17 to 64 rows, 1.1 to 1.25 of the other.
 
     Unreduced sums: up to 128 rows (at 256 the eight planes cost the next norm what the product gains), from K = 2048 on; for shorter
     ones the ranges of the split-K plan do as well or better (8 bits, 128 rows, 1000 x 1216 7.5 -> 9.6 us with the norm)."""

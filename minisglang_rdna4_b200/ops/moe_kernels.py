@@ -258,7 +258,8 @@ def quantise_sorted(kind: str, x, pair_row, rows: int, k: int):
 
 def few_rows_block(pairs: int, experts: int, two_inter: int, hidden: int) -> int:
     """Rows of a tile for ``gemm_fp8_block_few``, 0 where the 128-row tiles of ``gemm_fp8_block`` are taken: enough for the rows
-    that an expert has on average with room to spare (a second tile reads the expert's weights again, from L2). B200, 128
+    that an expert has on average (``pairs`` of the step over the ``experts`` here: where others have experts too, more than it has) with
+    room to spare (a second tile reads the expert's weights again, from L2). B200, 128
     experts of 2048 x 768, us a layer with tiles of 16 / 32 / 128 rows: 8 rows on average 137 / 149 / 179, 16 172 / 152 / 188, 20
     209 / 154 / 183, 32 273 / 199 / 189."""
     if two_inter % 256 or hidden % 128 or max(two_inter // 2, hidden) > 4096:
