@@ -92,8 +92,8 @@ def test_a_layer_in_both_forms():
         got = MK.moe_forward_quant("fp8_block", x, w, wt, ids)
         sp, pr, te, _ = MK.moe_align(ids, 0, e)
         want = MK._combine(MK.run_experts("fp8_block", MK._permute(x, sp, k), te, w, x.dtype), wt, pr, x, k)
-        # the same sums in the same order; an e4m3 or 16-bit value may round the other way
-        assert float((got.double() - want.double()).norm() / want.double().norm()) < 2.0 ** -8
+        # the same sums and roundings in the same order: a verification step, which has more rows, agrees with decode steps
+        assert torch.equal(got, want)
 
 
 def test_what_it_does_not_take():
